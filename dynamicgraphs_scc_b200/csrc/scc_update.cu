@@ -35,87 +35,167 @@ __global__ void k_upd_keys(int64_t k, const int32_t* __restrict__ a, const int32
     }
 }
 
-// For each deleted key (row, col): mark every copy of col in row's sorted list.
-__global__ void k_upd_mark_deleted(int64_t k, const unsigned long long* __restrict__ keys,
-                                   const int32_t* __restrict__ off, const int32_t* __restrict__ adj,
-                                   uint8_t* __restrict__ dead, int32_t* __restrict__ ndead) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < k; i += (int64_t)gridDim.x * blockDim.x) {
-        unsigned long long key = keys[i];
-        if (key == ~0ull || (i > 0 && keys[i - 1] == key)) continue;   // skip repeats of the same pair
-        int32_t r = (int32_t)(key >> 32), c = (int32_t)(uint32_t)key;
-        int32_t lo = off[r], hi = off[r + 1];
-        while (lo < hi) { int32_t mid = (lo + hi) >> 1; if (adj[mid] < c) lo = mid + 1; else hi = mid; }
-        int32_t cnt = 0;
-        for (int32_t e = lo; e < off[r + 1] && adj[e] == c; ++e) { dead[e] = 1; cnt++; }
-        if (cnt) atomicAdd(ndead + r, cnt);
+// The merge of one side (CSR or transpose) treats the adjacency array as one
+// ascending sequence of (row, col) keys.  A batch changes it at few places, so
+// an old entry only moves by a shift: the inserted keys placed before it minus
+// the deleted entries before it, constant between two neighbouring events.
+//   k_upd_events   where each event lies in the old array (a search per key)
+//   k_upd_offsets  the new offsets: the old ones shifted the same way
+//   k_upd_move     the old entries, copied with their shift
+//   k_upd_place    the inserted entries
+// Every kernel is balanced over entries, vertices or keys.  (One warp per list
+// took as long as the largest hub needed: 2.7 ms a side on R-MAT s22, whose
+// largest list has 95,000 entries, against 0.16 ms for the copy now; the copy
+// is bound by HBM at 4 B read and 4 B written per entry.)
+
+// The number of elements of a[0, k), ascending, that come before `key` (LE: that
+// are <= key), searched by the whole warp 33 ways at a time; the same in every lane.
+template <bool LE, typename T>
+__device__ __forceinline__ int64_t warp_count_before(const T* __restrict__ a, int64_t k, T key) {
+    const int lane = threadIdx.x & 31;
+    int64_t lo = 0, hi = k;
+    while (hi > lo) {
+        const int64_t step = (hi - lo + 32) / 33;           // 32 probes split [lo, hi) into 33 parts
+        const int64_t at = lo + step * (lane + 1) - 1;
+        bool before = false;
+        if (at < hi) { const T x = a[at]; before = LE ? x <= key : x < key; }
+        const int c = __popc(__ballot_sync(0xFFFFFFFFu, before));   // probes ascend: the true ones come first
+        lo += step * c;
+        if (c < 32) hi = min(hi, lo + step - 1);            // probe c did not come before
+    }
+    return lo;
+}
+
+// The same inside [lo, hi) for one thread.
+template <bool LE, typename T>
+__device__ __forceinline__ int32_t count_before(const T* __restrict__ a, int32_t lo, int32_t hi, T key) {
+    while (lo < hi) {
+        const int32_t mid = lo + ((hi - lo) >> 1);
+        const T x = __ldg(a + mid);
+        if (LE ? x <= key : x < key) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+
+// Places of the events in the old array.  A deleted key (row, col) is the run
+// of its copies, [run_lo, run_lo + run_cnt) (no copy: run_cnt 0); of repeats of
+// one key the last has the count, so that the last run starting at or before
+// an entry is the one that can cover it.  An inserted key goes behind the old
+// entries <= it.  Keys ascend, so run_lo and ins_at do too.
+__global__ void k_upd_events(int32_t kdel, const unsigned long long* __restrict__ del, int32_t kins,
+                             const unsigned long long* __restrict__ ins, const int32_t* __restrict__ off,
+                             const int32_t* __restrict__ adj, int32_t* __restrict__ run_lo,
+                             int32_t* __restrict__ run_cnt, int32_t* __restrict__ ins_at) {
+    const int64_t total = (int64_t)kdel + kins;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        if (i < kdel) {
+            const unsigned long long key = del[i];
+            const int32_t r = (int32_t)(key >> 32), c = (int32_t)(uint32_t)key;
+            const int32_t e = off[r + 1];
+            const int32_t lo = count_before<false>(adj, off[r], e, c);
+            int32_t cnt = 0;
+            if (!(i + 1 < kdel && del[i + 1] == key)) cnt = count_before<true>(adj, lo, e, c) - lo;
+            run_lo[i] = lo;
+            run_cnt[i] = cnt;
+        } else {
+            const unsigned long long key = ins[i - kdel];
+            const int32_t r = (int32_t)(key >> 32), c = (int32_t)(uint32_t)key;
+            ins_at[i - kdel] = count_before<true>(adj, off[r], off[r + 1], c);
+        }
     }
 }
 
-// new degree = old - dead + inserted
-__global__ void k_upd_degrees(int32_t n, const int32_t* __restrict__ off, const int32_t* __restrict__ ndead,
-                              const unsigned long long* __restrict__ ins, int64_t kins, int32_t* __restrict__ ins_begin,
-                              int32_t* __restrict__ deg) {
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-        // inserted keys of row v: [lower_bound(v<<32), lower_bound((v+1)<<32))
-        unsigned long long lo_key = (unsigned long long)v << 32;
-        int64_t lo = 0, hi = kins;
-        while (lo < hi) { int64_t mid = (lo + hi) >> 1; if (ins[mid] < lo_key) lo = mid + 1; else hi = mid; }
-        int64_t a = lo;
-        hi = kins;
-        unsigned long long hi_key = (unsigned long long)(v + 1) << 32;
-        while (lo < hi) { int64_t mid = (lo + hi) >> 1; if (ins[mid] < hi_key) lo = mid + 1; else hi = mid; }
-        ins_begin[v] = (int32_t)a;
-        deg[v] = (off[v + 1] - off[v]) - ndead[v] + (int32_t)(lo - a);
+// new_off[v] = off[v] + inserted keys of rows before v - deleted entries before
+// off[v].  A warp takes 128 consecutive offsets: it searches the batch for its
+// first and last one together, its lanes only between those two.
+#define UPD_OFFS 128
+__global__ void k_upd_offsets(int32_t n, const int32_t* __restrict__ off, int32_t kdel,
+                              const int32_t* __restrict__ run_lo, const int32_t* __restrict__ run_pref, int32_t kins,
+                              const unsigned long long* __restrict__ ins, int32_t* __restrict__ new_off) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t groups = ((int64_t)n + UPD_OFFS) / UPD_OFFS;          // n + 1 offsets
+    for (int64_t gi = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; gi < groups; gi += nwarps) {
+        const int64_t v0 = gi * UPD_OFFS, v1 = min((int64_t)n, v0 + UPD_OFFS - 1);
+        const int32_t i0 = (int32_t)warp_count_before<false>(ins, kins, (unsigned long long)v0 << 32);
+        const int32_t i1 = i0 + (int32_t)warp_count_before<false>(ins + i0, kins - i0, (unsigned long long)v1 << 32);
+        const int32_t d0 = (int32_t)warp_count_before<false>(run_lo, kdel, off[v0]);
+        const int32_t d1 = d0 + (int32_t)warp_count_before<false>(run_lo + d0, kdel - d0, off[v1]);
+        for (int64_t v = v0 + lane; v <= v1; v += 32) {
+            const int32_t o = off[v];
+            const int32_t i = i0 == i1 ? i0 : count_before<false>(ins, i0, i1, (unsigned long long)v << 32);
+            const int32_t d = d0 == d1 ? d0 : count_before<false>(run_lo, d0, d1, o);
+            new_off[v] = o + i - run_pref[d];
+        }
     }
 }
 
-// Per-vertex merge of the kept old entries and the inserted ones (both sorted).
-__global__ void k_upd_merge(int32_t n, const int32_t* __restrict__ off, const int32_t* __restrict__ adj,
-                            const uint8_t* __restrict__ dead, const int32_t* __restrict__ ndead,
-                            const unsigned long long* __restrict__ ins, const int32_t* __restrict__ ins_begin,
-                            const int32_t* __restrict__ new_off, int32_t* __restrict__ new_adj,
-                            int32_t* __restrict__ kp) {
-    int lane = threadIdx.x & 31;
-    int64_t wstride = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < n; w += wstride) {
-        int32_t v = (int32_t)w;
-        int32_t b = off[v], e = off[v + 1];
-        int32_t nb = new_off[v];
-        int32_t nins = (new_off[v + 1] - nb) - ((e - b) - ndead[v]);
-        if (nins == 0 && ndead[v] == 0) {            // unchanged list: coalesced copy
-            for (int32_t k = lane; k < e - b; k += 32) new_adj[nb + k] = adj[b + k];
+// Events at or before the first entry of each tile of UPD_TILE old entries, in
+// the insert and the delete list (one more for the end): the tile's own events
+// lie between its pair and the next one.
+#define UPD_ITEMS 16
+#define UPD_TILE (32 * UPD_ITEMS)
+__global__ void k_upd_bounds(int32_t m, int32_t kdel, const int32_t* __restrict__ run_lo, int32_t kins,
+                             const int32_t* __restrict__ ins_at, int32_t tiles, int2* __restrict__ bound) {
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t <= tiles; t += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t i = (int32_t)min((int64_t)m, t * UPD_TILE);
+        bound[t] = make_int2(count_before<true>(ins_at, 0, kins, i), count_before<true>(run_lo, 0, kdel, i));
+    }
+}
+
+// Old entries to their new places, a tile per warp.  A tile with no event is
+// one shifted copy; in the others each lane searches the tile's own events.  A
+// place outside the new array (only a list that was not sorted could give one)
+// is skipped.  The bounds come from their own launch: searched here, they put
+// four dependent loads before every tile (R-MAT s22, 65 M entries and 100,000
+// events, a side: 314 us with the searches and a block per 4,096 entries,
+// 159 us so).
+__global__ void __launch_bounds__(SCC_THREADS) k_upd_move(int32_t m, const int32_t* __restrict__ adj,
+                                                          const int32_t* __restrict__ run_lo,
+                                                          const int32_t* __restrict__ run_pref,
+                                                          const int32_t* __restrict__ ins_at, int32_t tiles,
+                                                          const int2* __restrict__ bound, int64_t new_m,
+                                                          int32_t* __restrict__ new_adj) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; t < tiles; t += nwarps) {
+        const int64_t t0 = t * UPD_TILE + lane;
+        int32_t x[UPD_ITEMS];
+#pragma unroll
+        for (int j = 0; j < UPD_ITEMS; ++j) x[j] = t0 + 32 * j < m ? __ldcs(adj + t0 + 32 * j) : 0;
+        const int2 b0 = __ldg(bound + t), b1 = __ldg(bound + t + 1);
+        const int32_t dead0 = __ldg(run_pref + b0.y);
+        // a run that started at or before the tile may reach into it
+        const bool covered = b0.y > 0 && (int64_t)__ldg(run_lo + b0.y - 1) + (dead0 - __ldg(run_pref + b0.y - 1)) > t * UPD_TILE;
+        if (b0.x == b1.x && b0.y == b1.y && !covered) {
+            const int64_t at = t0 + b0.x - dead0;
+#pragma unroll
+            for (int j = 0; j < UPD_ITEMS; ++j)
+                if (t0 + 32 * j < m && (uint64_t)(at + 32 * j) < (uint64_t)new_m) __stcs(new_adj + at + 32 * j, x[j]);
             continue;
         }
-        // Changed list, merged by the whole warp.  A kept old entry x lands at
-        // (kept entries before it) + (inserted entries < x); an inserted y at
-        // (its index) + (kept old entries <= y), so equal values keep old-first
-        // order.  kp[i] records the kept count before old position i.
-        const unsigned long long* iv = ins + ins_begin[v];
-        int32_t kept_base = 0;
-        for (int32_t i0 = b; i0 < e; i0 += 32) {
-            int32_t i = i0 + lane;
-            bool valid = i < e;
-            int32_t x = valid ? adj[i] : 0;
-            bool kept = valid && !dead[i];
-            unsigned bal = __ballot_sync(0xFFFFFFFFu, kept);
-            int32_t r = __popc(bal & ((1u << lane) - 1u));
-            if (valid) kp[i] = kept_base + r;
-            if (kept) {
-                int32_t lo = 0, hi = nins;
-                while (lo < hi) { int32_t mid = (lo + hi) >> 1; if ((int32_t)(uint32_t)iv[mid] < x) lo = mid + 1; else hi = mid; }
-                new_adj[nb + kept_base + r + lo] = x;
-            }
-            kept_base += __popc(bal);
+#pragma unroll
+        for (int j = 0; j < UPD_ITEMS; ++j) {
+            const int64_t i = t0 + 32 * j;
+            if (i >= m) continue;
+            const int32_t before = count_before<true>(ins_at, b0.x, b1.x, (int32_t)i);
+            const int32_t d = count_before<true>(run_lo, b0.y, b1.y, (int32_t)i);
+            const int32_t dead = __ldg(run_pref + d);
+            if (d > 0 && (int64_t)__ldg(run_lo + d - 1) + (dead - __ldg(run_pref + d - 1)) > i) continue;      // deleted
+            const int64_t at = i + before - dead;
+            if ((uint64_t)at < (uint64_t)new_m) __stcs(new_adj + at, x[j]);
         }
-        __syncwarp();
-        for (int32_t j = lane; j < nins; j += 32) {
-            int32_t y = (int32_t)(uint32_t)iv[j];
-            int32_t lo = b, hi = e;          // first old entry > y
-            while (lo < hi) { int32_t mid = (lo + hi) >> 1; if (adj[mid] <= y) lo = mid + 1; else hi = mid; }
-            int32_t before = (lo < e) ? kp[lo] : kept_base;
-            new_adj[nb + j + before] = y;
-        }
-        __syncwarp();
+    }
+}
+
+// Inserted entries: behind the old entries <= them and the inserted ones before them.
+__global__ void k_upd_place(int32_t kins, const unsigned long long* __restrict__ ins,
+                            const int32_t* __restrict__ ins_at, int32_t kdel, const int32_t* __restrict__ run_lo,
+                            const int32_t* __restrict__ run_pref, int64_t new_m, int32_t* __restrict__ new_adj) {
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < kins; j += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t at0 = ins_at[j];
+        const int64_t at = (int64_t)at0 + j - run_pref[count_before<false>(run_lo, 0, kdel, at0)];
+        if ((uint64_t)at < (uint64_t)new_m) new_adj[at] = (int32_t)(uint32_t)ins[j];
     }
 }
 
@@ -228,49 +308,86 @@ static int sorted_keys(int64_t k, const int32_t* d_a, const int32_t* d_b, int32_
     return scc_impl_sort_keys_u64(tmpk.as<unsigned long long>(), out.as<unsigned long long>(), k, 32 + hb, st);
 }
 
-// Merge one side (off/adj) with sorted deleted and inserted keys; returns new arrays.
-static int merge_side(int32_t n, int64_t m, const int32_t* off, const int32_t* adj, const unsigned long long* del,
-                      int64_t kdel, const unsigned long long* ins, int64_t kins, cudaStream_t st, int32_t** new_off,
-                      int32_t** new_adj, int64_t* new_m) {
-    DevBuf dead, ndead, insb, deg, kp;
-    SCC_TRY(alloc(kp, sizeof(int32_t) * (size_t)(m > 0 ? m : 1), st));
-    SCC_TRY(alloc(dead, (size_t)(m > 0 ? m : 1), st));
-    SCC_TRY(alloc(ndead, sizeof(int32_t) * (size_t)n, st));
-    SCC_TRY(alloc(insb, sizeof(int32_t) * (size_t)n, st));
-    SCC_TRY(alloc(deg, sizeof(int32_t) * ((size_t)n + 1), st));
-    SCC_CUDA(cudaMemsetAsync(dead.p, 0, (size_t)(m > 0 ? m : 1), st));
-    SCC_CUDA(cudaMemsetAsync(ndead.p, 0, sizeof(int32_t) * (size_t)n, st));
-    SCC_CUDA(cudaMemsetAsync(deg.p, 0, sizeof(int32_t) * ((size_t)n + 1), st));
-    if (kdel > 0) {
-        k_upd_mark_deleted<<<scc_blocks(kdel), SCC_THREADS, 0, st>>>(kdel, del, off, adj, dead.as<uint8_t>(),
-                                                                     ndead.as<int32_t>());
+// One side of the merge: where the batch's events lie in the old arrays, then
+// the new arrays (NULL until they are allocated; freed on `st` unless taken).
+struct MergeSide {
+    const int32_t* off; const int32_t* adj;
+    const unsigned long long* del; const unsigned long long* ins;
+    DevBuf run_lo, run_pref, ins_at;
+    int32_t* new_off = nullptr; int32_t* new_adj = nullptr;
+    cudaStream_t st = nullptr;
+    int32_t dead = 0;               // entries deleted (valid after a synchronisation)
+    ~MergeSide() {
+        if (new_off) cudaFreeAsync(new_off, st);
+        if (new_adj) cudaFreeAsync(new_adj, st);
+    }
+};
+
+static int merge_events(MergeSide& x, int32_t kdel, int32_t kins, cudaStream_t st) {
+    DevBuf cnt;
+    x.st = st;
+    SCC_TRY(alloc(x.run_lo, sizeof(int32_t) * (size_t)kdel, st));
+    SCC_TRY(alloc(cnt, sizeof(int32_t) * ((size_t)kdel + 1), st));
+    SCC_TRY(alloc(x.run_pref, sizeof(int32_t) * ((size_t)kdel + 1), st));
+    SCC_TRY(alloc(x.ins_at, sizeof(int32_t) * (size_t)kins, st));
+    // one extra zero count: its exclusive prefix is the number of deleted entries
+    SCC_CUDA(cudaMemsetAsync(cnt.as<int32_t>() + kdel, 0, sizeof(int32_t), st));
+    if (kdel + kins > 0) {
+        k_upd_events<<<scc_blocks((int64_t)kdel + kins), SCC_THREADS, 0, st>>>(
+            kdel, x.del, kins, x.ins, x.off, x.adj, x.run_lo.as<int32_t>(), cnt.as<int32_t>(), x.ins_at.as<int32_t>());
         SCC_CUDA(cudaPeekAtLastError());
     }
-    if (n > 0) {
-        k_upd_degrees<<<scc_blocks(n), SCC_THREADS, 0, st>>>(n, off, ndead.as<int32_t>(), ins, kins, insb.as<int32_t>(),
-                                                             deg.as<int32_t>());
+    SCC_TRY(scc_impl_scan_i32(cnt.as<int32_t>(), x.run_pref.as<int32_t>(), (int64_t)kdel + 1, false, st));
+    SCC_CUDA(cudaMemcpyAsync(&x.dead, x.run_pref.as<int32_t>() + kdel, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    return SCC_OK;
+}
+
+static int merge_write(MergeSide& x, int32_t n, int64_t m, int32_t kdel, int32_t kins, cudaStream_t st) {
+    const int64_t new_m = m + kins - x.dead;
+    SCC_CUDA(scc_impl_malloc_async((void**)&x.new_off, sizeof(int32_t) * ((size_t)n + 1), st));
+    SCC_CUDA(scc_impl_malloc_async((void**)&x.new_adj, sizeof(int32_t) * (size_t)(new_m > 0 ? new_m : 1), st));
+    k_upd_offsets<<<scc_blocks(((int64_t)n / UPD_OFFS + 1) * 32, SCC_THREADS, 148 * 8), SCC_THREADS, 0, st>>>(
+        n, x.off, kdel, x.run_lo.as<int32_t>(), x.run_pref.as<int32_t>(), kins, x.ins, x.new_off);
+    SCC_CUDA(cudaPeekAtLastError());
+    if (m > 0) {
+        const int32_t tiles = (int32_t)((m + UPD_TILE - 1) / UPD_TILE);
+        DevBuf bound;
+        SCC_TRY(alloc(bound, sizeof(int2) * ((size_t)tiles + 1), st));
+        k_upd_bounds<<<scc_blocks((int64_t)tiles + 1), SCC_THREADS, 0, st>>>(
+            (int32_t)m, kdel, x.run_lo.as<int32_t>(), kins, x.ins_at.as<int32_t>(), tiles, bound.as<int2>());
+        SCC_CUDA(cudaPeekAtLastError());
+        k_upd_move<<<scc_blocks((int64_t)tiles * 32), SCC_THREADS, 0, st>>>(
+            (int32_t)m, x.adj, x.run_lo.as<int32_t>(), x.run_pref.as<int32_t>(), x.ins_at.as<int32_t>(), tiles,
+            bound.as<int2>(), new_m, x.new_adj);
         SCC_CUDA(cudaPeekAtLastError());
     }
-    int32_t* noff = nullptr;
-    SCC_CUDA(scc_impl_malloc_async((void**)&noff, sizeof(int32_t) * ((size_t)n + 1), st));
-    {
-        int rc = scc_impl_scan_i32(deg.as<int32_t>(), noff, (int64_t)n + 1, false, st);
-        if (rc != SCC_OK) { cudaFreeAsync(noff, st); return rc; }
+    if (kins > 0) {
+        k_upd_place<<<scc_blocks(kins), SCC_THREADS, 0, st>>>(kins, x.ins, x.ins_at.as<int32_t>(), kdel,
+                                                             x.run_lo.as<int32_t>(), x.run_pref.as<int32_t>(), new_m,
+                                                             x.new_adj);
+        SCC_CUDA(cudaPeekAtLastError());
     }
-    int32_t nm = 0;
-    SCC_CUDA(cudaMemcpyAsync(&nm, noff + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    return SCC_OK;
+}
+
+// Merge a batch (sorted keys of the CSR, and of the transpose) into g's arrays.
+// A failure leaves g as it was.
+static int merge_batch(scc_graph* g, const unsigned long long* del, const unsigned long long* del_t, int64_t kdel,
+                       const unsigned long long* ins, const unsigned long long* ins_t, int64_t kins, cudaStream_t st) {
+    MergeSide f, r;
+    f.off = g->begin; f.adj = g->node_idx; f.del = del; f.ins = ins;
+    r.off = g->r_begin; r.adj = g->r_node_idx; r.del = del_t; r.ins = ins_t;
+    SCC_TRY(merge_events(f, (int32_t)kdel, (int32_t)kins, st));
+    SCC_TRY(merge_events(r, (int32_t)kdel, (int32_t)kins, st));
     SCC_CUDA(cudaStreamSynchronize(st));
-    int32_t* nadj = nullptr;
-    cudaError_t e = scc_impl_malloc_async((void**)&nadj, sizeof(int32_t) * (size_t)(nm > 0 ? nm : 1), st);
-    if (e != cudaSuccess) { cudaFreeAsync(noff, st); return scc_cuda_status(e, "scratch allocation", __FILE__, __LINE__); }
-    if (n > 0) {
-        k_upd_merge<<<scc_blocks((int64_t)n * 32, SCC_THREADS, 148 * 16), SCC_THREADS, 0, st>>>(
-            n, off, adj, dead.as<uint8_t>(), ndead.as<int32_t>(), ins, insb.as<int32_t>(), noff, nadj,
-            kp.as<int32_t>());
-        SCC_CUDA(cudaPeekAtLastError());
-    }
-    SCC_CUDA(cudaStreamSynchronize(st));
-    *new_off = noff; *new_adj = nadj; *new_m = nm;
+    SCC_TRY(merge_write(f, g->n, g->m, (int32_t)kdel, (int32_t)kins, st));
+    SCC_TRY(merge_write(r, g->n, g->m, (int32_t)kdel, (int32_t)kins, st));
+    release_graph_arrays(g, st);
+    g->begin = f.new_off; g->node_idx = f.new_adj; g->r_begin = r.new_off; g->r_node_idx = r.new_adj;
+    f.new_off = f.new_adj = r.new_off = r.new_adj = nullptr;
+    g->m = g->m + kins - f.dead;
+    g->self_loops = -1;
+    g->async_arrays = true;
     return SCC_OK;
 }
 
@@ -291,6 +408,21 @@ static RoundArgs update_round_args(const scc_graph* g, scc_state* s) {
     a.cta_deg = s->tune.cta_deg;
     round_args_adjacency(a, g->node_idx, g->r_node_idx, g->m);
     return a;
+}
+
+// Decompose the classes an update left live (colours in [0, n), live list not
+// built).  The first round takes them as they are: they come from old SCCs, so
+// nearly all of one is still strongly connected, and pivoting it at once costs
+// less than peeling and splitting it first; what it leaves is peeled and split by
+// the next round.  Fresh colours must lie above every class colour.
+static int resolve_update(const scc_graph* g, scc_state* s) {
+    s->fresh = false;
+    s->prefinished = false;
+    s->live_count = -1;
+    const int32_t last = g->n - 1;
+    SCC_CUDA(cudaMemcpyAsync(s->ctr + CTR_NEXT_COLOR, &last, sizeof(int32_t), cudaMemcpyHostToDevice, s->stream));
+    s->h_ctr[CTR_NEXT_COLOR] = last;
+    return scc_impl_resolve_all(g, s, true);
 }
 
 static double ev_ms(cudaEvent_t a, cudaEvent_t b) {
@@ -344,17 +476,8 @@ extern "C" int scc_update_batch(scc_graph* g, scc_state* s, int64_t n_ins, const
     SCC_REQUIRE(!hbad, SCC_ERR_INVALID, "batch edge endpoint outside [0, %d)", n);
 
     // 1. CSR merge, both sides
-    int32_t *nb = nullptr, *na = nullptr, *nrb = nullptr, *nra = nullptr;
-    int64_t m1 = 0, m2 = 0;
-    SCC_TRY(merge_side(n, g->m, g->begin, g->node_idx, del_k.as<unsigned long long>(), n_del,
-                       ins_k.as<unsigned long long>(), n_ins, st, &nb, &na, &m1));
-    int rc = merge_side(n, g->m, g->r_begin, g->r_node_idx, del_t.as<unsigned long long>(), n_del,
-                        ins_t.as<unsigned long long>(), n_ins, st, &nrb, &nra, &m2);
-    if (rc != SCC_OK) { cudaFreeAsync(nb, st); cudaFreeAsync(na, st); return rc; }
-    release_graph_arrays(g, st);
-    g->begin = nb; g->node_idx = na; g->r_begin = nrb; g->r_node_idx = nra; g->m = m1;
-    g->self_loops = -1;
-    g->async_arrays = true;
+    SCC_TRY(merge_batch(g, del_k.as<unsigned long long>(), del_t.as<unsigned long long>(), n_del,
+                        ins_k.as<unsigned long long>(), ins_t.as<unsigned long long>(), n_ins, st));
     SCC_CUDA(cudaEventRecord(s->ev[9], st));
 
     // 2. deletions: re-decompose the SCCs that lost an internal edge
@@ -370,12 +493,7 @@ extern "C" int scc_update_batch(scc_graph* g, scc_state* s, int64_t n_ins, const
         SCC_LAUNCHED(s);
         SCC_TRY(scc_sync_counters(s));
         out.affected_delete = s->h_ctr[CTR_SPARE0];
-        if (out.affected_delete > 0) {
-            s->fresh = false;
-            s->prefinished = false;
-            s->live_count = -1;
-            SCC_TRY(scc_impl_resolve_all(g, s));
-        }
+        if (out.affected_delete > 0) SCC_TRY(resolve_update(g, s));
     }
     SCC_CUDA(cudaEventRecord(s->ev[10], st));
 
@@ -406,7 +524,7 @@ extern "C" int scc_update_batch(scc_graph* g, scc_state* s, int64_t n_ins, const
             s->fresh = false;
             s->prefinished = false;
             s->live_count = -1;
-            if (out.affected_insert > 0) SCC_TRY(scc_impl_resolve_all(g, s));
+            if (out.affected_insert > 0) SCC_TRY(resolve_update(g, s));
         } else {
             k_upd_fill<<<scc_blocks(n), SCC_THREADS, 0, st>>>(n, s->color, SCC_COLOR_DONE);
             SCC_LAUNCHED(s);
@@ -442,8 +560,6 @@ extern "C" int scc_decremental_delete(scc_graph* g, scc_state* s, int64_t n_del,
 extern "C" int scc_insert_idea1(scc_graph* g, scc_state* s, int64_t n_ins, const int32_t* src, const int32_t* dst,
                                 scc_run_stats* stats) {
     SCC_REQUIRE(g && s, SCC_ERR_INVALID, "NULL argument");
-    int32_t *nb = nullptr, *na = nullptr, *nrb = nullptr, *nra = nullptr;
-    int64_t m1 = 0, m2 = 0;
     SCC_CUDA(cudaSetDevice(s->device));
     cudaStream_t st = s->stream;
     DevBuf d_s, d_d, bad, ins_k, ins_t;
@@ -460,14 +576,8 @@ extern "C" int scc_insert_idea1(scc_graph* g, scc_state* s, int64_t n_ins, const
     SCC_CUDA(cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     SCC_CUDA(cudaStreamSynchronize(st));
     SCC_REQUIRE(!hbad, SCC_ERR_INVALID, "inserted edge endpoint outside [0, %d)", g->n);
-    SCC_TRY(merge_side(g->n, g->m, g->begin, g->node_idx, nullptr, 0, ins_k.as<unsigned long long>(), n_ins, st, &nb,
-                       &na, &m1));
-    SCC_TRY(merge_side(g->n, g->m, g->r_begin, g->r_node_idx, nullptr, 0, ins_t.as<unsigned long long>(), n_ins, st,
-                       &nrb, &nra, &m2));
-    release_graph_arrays(g, st);
-    g->begin = nb; g->node_idx = na; g->r_begin = nrb; g->r_node_idx = nra; g->m = m1;
-    g->self_loops = -1;
-    g->async_arrays = true;
+    SCC_TRY(merge_batch(g, nullptr, nullptr, 0, ins_k.as<unsigned long long>(), ins_t.as<unsigned long long>(), n_ins,
+                        st));
     SCC_TRY(scc_state_reset(s));
     return scc_run(g, s, SCC_METHOD_GLOBAL_WCC_FB, SCC_PIVOT_DEGREE, stats);
 }
