@@ -1,8 +1,9 @@
 // Batched decomposition of many independent small graphs in ONE persistent
 // launch: each block takes whole graphs from a device counter (largest
-// first) and runs the complete method on each inside the block -- Trim1 to
-// the fixpoint, then rounds of pivot / FW+BW reachability / classify / peel
-// over every class of that graph at once (the structure of
+// first) and runs the complete method on each inside the block -- a first
+// round of FW-BW from one pivot with its marks in shared memory, then Trim1 to the
+// fixpoint and rounds of pivot / FW+BW reachability / classify / peel
+// over every class left of that graph at once (the structure of
 // do_baseline_global_wcc_fb and start_workers_fw_bw, src/scc_main.cc:272-351,
 // src/scc_fb_seq2.cc:292-351) -- with __syncthreads between the steps instead
 // of kernel boundaries and host round trips.  One launch per batch, so the
@@ -34,6 +35,9 @@ struct BatchArgs {
     int32_t* ctr;               // BATCH_CTR_* counters
     int32_t warp_deg;           // lists longer than this are expanded by a whole warp
     const int32_t* members;     // class mode: unit k is members[offs[k] .. offs[k+1]); NULL: vertex ids
+    int32_t marks_cap;          // graphs of at most this many vertices keep the first round's marks in shared memory
+    int32_t vec_adj;            // both adjacency arrays start on a 16-byte boundary
+    int64_t adj_len;            // their entries
 };
 
 __device__ __forceinline__ int32_t b_fw_colour(int32_t p) { return 3 * p + 1; }
@@ -170,6 +174,7 @@ __device__ void b_peel(const BatchArgs& a, int32_t* q, int32_t* qc, int32_t* s_t
     while (true) {
         int32_t t = *s_tail;
         if (t > cap) t = cap;
+        __syncthreads();          // every warp has read the tail before one appends
         if (h >= t) break;
         for (int32_t base = h + wid * 32; base < t; base += nwarps * 32) {
             int32_t i = base + lane;
@@ -220,8 +225,295 @@ __device__ void b_peel(const BatchArgs& a, int32_t* q, int32_t* qc, int32_t* s_t
     }
 }
 
+// ------------------------------------------------------------------ a graph's first round
+// A whole graph is one class, so its first FW-BW round needs no colours: mark
+// bytes in shared memory replace the marks and the colour gathers in global
+// memory, and the round comes before the peel, which then only sees what the
+// round left.  Narrow frontiers are expanded top down from the queue; from a
+// quarter of the vertices on, a sweep over all vertices takes over, whose
+// offsets and lists are read in order.  Bound by instruction issue and by the
+// round trips of narrow levels.
+// 4,096 graphs, 63.8 M vertices, 383 M edges, default shape: 23.7 ms with
+// colours and marks in global memory and the peel first, 3.7 ms so (sweeps
+// from a sixteenth on 3.8 ms, from half on 4.4 ms).
+#define B_BLOCK_DEG 512          // top-down lists longer than this are expanded by the whole block
+#define B_BIG 64                 // such items one level sets aside (further ones: by their warp)
+#define B_SWEEP 4                // sweep once the frontier (both directions) is this share of the vertices not reached
+#define B_STEP 8                 // entries of a short list claimed together
+#define B_PROBES 8               // two-chunk probes a lane makes alone before the warp takes the list
+
+struct FirstRound {
+    volatile uint8_t* marks;     // bit 0 FW reached, bit 1 BW reached, of vertex lo + i
+    int32_t lo, ng;
+};
+
+// An id outside the graph (a batch whose graphs are not closed) is not claimed.
+__device__ __forceinline__ bool b_claim(const FirstRound& r, int dir, int32_t u) {
+    const uint32_t i = (uint32_t)(u - r.lo), bit = 1u << dir;
+    if (i >= (uint32_t)r.ng || (r.marks[i] & bit)) return false;
+    const uint32_t sh = (i & 3u) * 8u;
+    return !((atomicOr(reinterpret_cast<uint32_t*>(const_cast<uint8_t*>(r.marks) + (i & ~3u)), bit << sh) >> sh) & bit);
+}
+
+// Is one of the four entries u at adj[c], ... that lie in [k, e) reached (bit of its mark)?
+__device__ __forceinline__ bool b_hit4(const FirstRound& r, uint32_t bit, const int4& u, int32_t c, int32_t k, int32_t e) {
+    const int32_t x[4] = {u.x, u.y, u.z, u.w};
+    uint32_t m = 0u;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t i = (uint32_t)(x[j] - r.lo);
+        if ((uint32_t)(c + j - k) < (uint32_t)(e - k) && i < (uint32_t)r.ng) m |= r.marks[i];
+    }
+    return m & bit;
+}
+
+__device__ __forceinline__ int4 b_load4(const BatchArgs& a, const int32_t* __restrict__ adj, int32_t c) {
+    if (a.vec_adj && (int64_t)c + 4 <= a.adj_len) return __ldg(reinterpret_cast<const int4*>(adj + c));
+    int4 x;      // the array's last entries, or arrays that are not 16-byte aligned
+    x.x = c < a.adj_len ? __ldg(adj + c) : 0;
+    x.y = c + 1 < a.adj_len ? __ldg(adj + c + 1) : 0;
+    x.z = c + 2 < a.adj_len ? __ldg(adj + c + 2) : 0;
+    x.w = c + 3 < a.adj_len ? __ldg(adj + c + 3) : 0;
+    return x;
+}
+
+// Lists still open after a lane's own probes, by the whole warp, 32 entries at a time.
+__device__ __forceinline__ bool b_probe_long(const FirstRound& r, uint32_t bit, const int32_t* __restrict__ adj,
+                                             int32_t k, int32_t e) {
+    const unsigned full = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    bool hit = false;
+    unsigned open = __ballot_sync(full, k < e);
+    while (open) {
+        const int l = __ffs(open) - 1;
+        open &= open - 1;
+        const int32_t lk = __shfl_sync(full, k, l), le = __shfl_sync(full, e, l);
+        bool found = false;
+        for (int32_t j0 = lk; j0 < le && !found; j0 += 32) {
+            const int32_t j = j0 + lane;
+            const uint32_t i = j < le ? (uint32_t)(__ldg(adj + j) - r.lo) : UINT32_MAX;
+            found = __any_sync(full, i < (uint32_t)r.ng && (r.marks[i] & bit));
+        }
+        if (lane == l) hit = found;
+    }
+    return hit;
+}
+
+// One sweep over the n vertices of `list` (places in the graph; NULL: all of
+// them): each one not yet reached looks for a reached in-neighbour (FW) and a
+// reached out-neighbour (BW); what it finds joins the queue, and the vertices still
+// not reached both ways are listed in `open` for the next sweep, so a sweep
+// costs what the one before it left.  A lane per vertex, two aligned int4
+// chunks of each direction's list in flight at once (a list of six entries is
+// then done in one round trip after its offsets), a list left at its first hit.
+// Bound by instruction issue and the round trips of a vertex's loads.  On the
+// batch named above: 3.7 ms; all vertices in every sweep 4.4 ms; the
+// lists of 32 vertices read end to end, a row of 32 entries at a time 5.7 ms; one
+// chunk and one direction at a time 7.1 ms.
+__device__ void b_sweep(const BatchArgs& a, const FirstRound& r, const int32_t* list, int32_t n, int32_t* open,
+                        int32_t* s_open, int32_t* q, int32_t* s_tail) {
+    const unsigned full = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    for (int32_t at0 = (int32_t)threadIdx.x - lane; at0 < n; at0 += (int32_t)blockDim.x) {
+        const bool in = at0 + lane < n;
+        const int32_t i = !in ? 0 : list ? list[at0 + lane] : at0 + lane;
+        const int32_t v = r.lo + i;
+        const uint32_t had = in ? r.marks[i] : 3u;
+        int32_t k0 = 0, e0 = 0, k1 = 0, e1 = 0;
+        if (!(had & 1u)) { k0 = __ldg(a.rbegin + v); e0 = __ldg(a.rbegin + v + 1); }
+        if (!(had & 2u)) { k1 = __ldg(a.begin + v); e1 = __ldg(a.begin + v + 1); }
+        bool hit0 = false, hit1 = false;
+        for (int t = 0; t < B_PROBES && (k0 < e0 || k1 < e1); ++t) {
+            const int32_t c0 = k0 & ~3, c1 = k1 & ~3;
+            int4 x0 = {0, 0, 0, 0}, x1 = x0, y0 = x0, y1 = x0;
+            if (k0 < e0) x0 = b_load4(a, a.radj, c0);
+            if (c0 + 4 < e0) x1 = b_load4(a, a.radj, c0 + 4);
+            if (k1 < e1) y0 = b_load4(a, a.adj, c1);
+            if (c1 + 4 < e1) y1 = b_load4(a, a.adj, c1 + 4);
+            if (k0 < e0) {
+                hit0 = b_hit4(r, 1u, x0, c0, k0, e0) || b_hit4(r, 1u, x1, c0 + 4, k0, e0);
+                k0 = hit0 ? e0 : c0 + 8;
+            }
+            if (k1 < e1) {
+                hit1 = b_hit4(r, 2u, y0, c1, k1, e1) || b_hit4(r, 2u, y1, c1 + 4, k1, e1);
+                k1 = hit1 ? e1 : c1 + 8;
+            }
+        }
+        __syncwarp();
+        hit0 = b_probe_long(r, 1u, a.radj, k0, e0) || hit0;
+        hit1 = b_probe_long(r, 2u, a.adj, k1, e1) || hit1;
+        // the sweep alone writes marks now, each by its own lane
+        const uint32_t now = had | (hit0 ? 1u : 0u) | (hit1 ? 2u : 0u);
+        if (now != had) r.marks[i] = (uint8_t)now;
+        const unsigned n0 = __ballot_sync(full, hit0), n1 = __ballot_sync(full, hit1), no = __ballot_sync(full, now != 3u);
+        int32_t at = 0, oat = 0;
+        if (lane == 0) {
+            if (n0 | n1) at = atomicAdd(s_tail, __popc(n0) + __popc(n1));
+            if (no) oat = atomicAdd(s_open, __popc(no));
+        }
+        at = __shfl_sync(full, at, 0);
+        oat = __shfl_sync(full, oat, 0);
+        // a vertex enters at most once per direction, so the queue never passes 2 ng
+        if (hit0) q[at + __popc(n0 & lt)] = v;
+        if (hit1) q[at + __popc(n0) + __popc(n1 & lt)] = v | (1 << DIR_SHIFT);
+        if (now != 3u) open[oat + __popc(no & lt)] = i;
+    }
+}
+
+// One top-down level: the items q[h, t).
+__device__ void b_expand(const BatchArgs& a, const FirstRound& r, int32_t* q, int32_t h, int32_t t, int32_t* s_tail,
+                         int32_t* s_big, int32_t* s_nbig, int32_t cap) {
+    const unsigned full = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5, wid = threadIdx.x >> 5;
+    int32_t* err = a.ctr + BATCH_CTR_ERROR;
+    for (int32_t base = h + wid * 32; base < t; base += nwarps * 32) {
+        const int32_t i = base + lane;
+        const bool valid = i < t;
+        const int32_t it = valid ? q[i] : 0;
+        const int32_t v = it & ITEM_MASK, dir = (it >> DIR_SHIFT) & 1;
+        const int32_t* off = dir ? a.rbegin : a.begin;
+        const int32_t b = valid ? __ldg(off + v) : 0;
+        int32_t e = valid ? __ldg(off + v + 1) : 0;
+        if (e - b > B_BLOCK_DEG) {
+            const int32_t at = atomicAdd(s_nbig, 1);
+            if (at < B_BIG) { s_big[at] = it; e = b; }
+        }
+        unsigned big = __ballot_sync(full, e - b > a.warp_deg);
+        while (big) {
+            const int l = __ffs(big) - 1;
+            big &= big - 1;
+            const int32_t lb = __shfl_sync(full, b, l), le = __shfl_sync(full, e, l), ld = __shfl_sync(full, dir, l);
+            const int32_t* adj = ld ? a.radj : a.adj;
+            for (int32_t j0 = lb; j0 < le; j0 += 32) {
+                const int32_t j = j0 + lane;
+                const int32_t u = j < le ? __ldg(adj + j) : 0;
+                b_append(j < le && b_claim(r, ld, u), u | (ld << DIR_SHIFT), q, s_tail, cap, err);
+            }
+        }
+        const int32_t mydeg = e - b <= a.warp_deg ? e - b : 0;
+        const int32_t maxd = (int32_t)__reduce_max_sync(full, (unsigned)mydeg);
+        const int32_t* adj = dir ? a.radj : a.adj;
+        // eight entries of every lane's list at a time: loads, then claims, then one
+        // append for all of them
+        for (int32_t j0 = 0; j0 < maxd; j0 += B_STEP) {
+            int32_t u[B_STEP];
+            unsigned got[B_STEP];
+            int32_t total = 0;
+#pragma unroll
+            for (int j = 0; j < B_STEP; ++j) u[j] = j0 + j < mydeg ? __ldg(adj + b + j0 + j) : 0;
+#pragma unroll
+            for (int j = 0; j < B_STEP; ++j) {
+                got[j] = __ballot_sync(full, j0 + j < mydeg && b_claim(r, dir, u[j]));
+                total += __popc(got[j]);
+            }
+            if (total == 0) continue;
+            int32_t at = 0;
+            if (lane == 0) at = atomicAdd(s_tail, total);
+            at = __shfl_sync(full, at, 0);
+            // claimed once per direction, so the queue never passes 2 ng
+#pragma unroll
+            for (int j = 0; j < B_STEP; ++j) {
+                if ((got[j] >> lane) & 1u) q[at + __popc(got[j] & ((1u << lane) - 1u))] = u[j] | (dir << DIR_SHIFT);
+                at += __popc(got[j]);
+            }
+        }
+    }
+    __syncthreads();
+    const int32_t nbig = min(*s_nbig, B_BIG);
+    for (int32_t x = 0; x < nbig; ++x) {
+        const int32_t it = s_big[x], v = it & ITEM_MASK, dir = (it >> DIR_SHIFT) & 1;
+        const int32_t* off = dir ? a.rbegin : a.begin;
+        const int32_t* adj = dir ? a.radj : a.adj;
+        const int32_t b = __ldg(off + v), e = __ldg(off + v + 1);
+        for (int32_t j0 = b; j0 < e; j0 += (int32_t)blockDim.x) {
+            const int32_t j = j0 + (int32_t)threadIdx.x;
+            const int32_t u = j < e ? __ldg(adj + j) : 0;
+            b_append(j < e && b_claim(r, dir, u), u | (dir << DIR_SHIFT), q, s_tail, cap, err);
+        }
+    }
+}
+
+// The first round of the graph [lo, lo + ng): colours and components of all its
+// vertices are written, those it did not resolve are listed in live.  Returns
+// their number.  s: 64 ints, s_big: B_BIG ints, marks: ng bytes rounded up to words.
+__device__ int32_t b_first_round(const BatchArgs& a, int32_t lo, int32_t ng, int32_t c0, int32_t* s, int32_t* s_big,
+                                 uint32_t* marks, int32_t* q, int32_t* live, int32_t* live2, int32_t* levels) {
+    const unsigned full = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    int32_t* s_tail = s;
+    int32_t* s_nbig = s + 1;
+    unsigned long long* s_key = reinterpret_cast<unsigned long long*>(s + 2);
+    int32_t* s_open = s + 4;
+    FirstRound r;
+    r.marks = reinterpret_cast<uint8_t*>(marks); r.lo = lo; r.ng = ng;
+    for (int32_t i = threadIdx.x; i < (ng + 3) >> 2; i += blockDim.x) marks[i] = 0u;
+    if (threadIdx.x == 0) { *s_key = 0ull; *s_nbig = 0; *s_open = 0; }
+    __syncthreads();
+    unsigned long long best = 0ull;
+#pragma unroll 4
+    for (int32_t i = threadIdx.x; i < ng; i += blockDim.x) {
+        const unsigned long long k = pivot_key(a.begin, a.rbegin, lo + i);
+        best = k > best ? k : best;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long y = __shfl_xor_sync(full, best, o);
+        best = y > best ? y : best;
+    }
+    if (lane == 0) atomicMax(s_key, best);
+    __syncthreads();
+    const int32_t p = pivot_unhash((uint32_t)*s_key);
+    if (threadIdx.x == 0) {
+        r.marks[p - lo] = 3;
+        q[0] = p;
+        q[1] = p | (1 << DIR_SHIFT);
+        *s_tail = 2;
+    }
+    __syncthreads();
+    int32_t h = 0;
+    const int32_t* list = nullptr;      // what the last sweep left open (NULL: no sweep yet)
+    int32_t nopen = ng;
+    while (true) {
+        const int32_t t = min(*s_tail, 2 * ng);
+        __syncthreads();          // every warp has read the tail before one appends
+        if (h >= t) break;
+        ++*levels;
+        if ((t - h) * (int64_t)B_SWEEP >= nopen) {
+            int32_t* out = list == live ? live2 : live;
+            b_sweep(a, r, list, nopen, out, s_open, q, s_tail);
+            __syncthreads();
+            list = out;
+            nopen = *s_open;
+            __syncthreads();
+            if (threadIdx.x == 0) *s_open = 0;
+        } else {
+            b_expand(a, r, q, h, t, s_tail, s_big, s_nbig, 2 * ng);
+            __syncthreads();
+            if (threadIdx.x == 0) *s_nbig = 0;
+        }
+        h = t;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *s_tail = 0;
+    __syncthreads();
+    for (int32_t i0 = threadIdx.x - lane; i0 < ng; i0 += blockDim.x) {
+        const int32_t i = i0 + lane, v = lo + i;
+        const uint32_t m = i < ng ? r.marks[i] : 3u;
+        if (i < ng) {
+            a.scc[v] = m == 3u ? p : SCC_NIL_NODE;
+            a.color[v] = m == 3u ? SCC_COLOR_DONE : m == 1u ? b_fw_colour(p) : m == 2u ? b_bw_colour(p) : c0;
+            if (m != 3u) a.mark[v] = 0;
+        }
+        b_append(m != 3u, v, live, s_tail, ng, a.ctr + BATCH_CTR_ERROR);
+    }
+    __syncthreads();
+    const int32_t left = *s_tail;
+    __syncthreads();
+    return left;
+}
+
 // ------------------------------------------------------------------ one graph
-__device__ void b_graph(const BatchArgs& a, int32_t gi, int32_t* s) {
+__device__ void b_graph(const BatchArgs& a, int32_t gi, int32_t* s, int32_t* s_big, uint32_t* marks) {
     int32_t* s_tail = s;          // queue tail
     int32_t* s_warp = s + 32;     // scan scratch (32 ints)
     const int32_t lo = a.offs[gi], hi = a.offs[gi + 1];
@@ -233,17 +525,22 @@ __device__ void b_graph(const BatchArgs& a, int32_t gi, int32_t* s) {
     // one class per unit: colour 3 x its first vertex (a multiple of 3, so it
     // never meets the 3p+1 / 3p+2 colours of a pivot's parts)
     const int32_t c0 = 3 * (a.members ? a.members[lo] : lo);
-    for (int32_t i = threadIdx.x; i < ng; i += blockDim.x) {
-        int32_t v = a.members ? a.members[lo + i] : lo + i;
-        a.color[v] = c0;
-        a.scc[v] = SCC_NIL_NODE;
-        a.mark[v] = 0;
-        live[i] = v;
-    }
     int32_t nlive = ng;
     int32_t rounds = 0, levels = 0;
-    __syncthreads();
-    while (true) {
+    if (!a.members && ng <= a.marks_cap) {
+        nlive = b_first_round(a, lo, ng, c0, s, s_big, marks, q, live, live2, &levels);
+        rounds = 1;
+    } else {
+        for (int32_t i = threadIdx.x; i < ng; i += blockDim.x) {
+            int32_t v = a.members ? a.members[lo + i] : lo + i;
+            a.color[v] = c0;
+            a.scc[v] = SCC_NIL_NODE;
+            a.mark[v] = 0;
+            live[i] = v;
+        }
+        __syncthreads();
+    }
+    while (nlive > 0) {
         // peel inside the classes
         if (threadIdx.x == 0) *s_tail = 0;
         __syncthreads();
@@ -295,6 +592,7 @@ __device__ void b_graph(const BatchArgs& a, int32_t gi, int32_t* s) {
         const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5, wid = threadIdx.x >> 5;
         while (true) {
             int32_t t = min(*s_tail, 2 * ng);
+            __syncthreads();      // every warp has read the tail before one appends
             if (h >= t) break;
             ++levels;
             for (int32_t base = h + wid * 32; base < t; base += nwarps * 32) {
@@ -368,9 +666,11 @@ __device__ void b_graph(const BatchArgs& a, int32_t gi, int32_t* s) {
     __syncthreads();
 }
 
-__global__ void k_batch_scc(BatchArgs a) {
-    __shared__ int32_t s[64];
+__global__ void __launch_bounds__(1024, 1) k_batch_scc(BatchArgs a) {
+    __shared__ __align__(8) int32_t s[64];
+    __shared__ int32_t s_big[B_BIG];
     __shared__ int32_t s_gi;
+    extern __shared__ uint32_t s_marks[];
     while (true) {
         if (threadIdx.x == 0) {
             // a device error anywhere ends every block (read by one thread, so the block agrees)
@@ -380,7 +680,7 @@ __global__ void k_batch_scc(BatchArgs a) {
         int32_t k = s_gi;
         __syncthreads();
         if (k >= a.G) break;
-        b_graph(a, a.order[k], s);
+        b_graph(a, a.order[k], s, s_big, s_marks);
     }
 }
 
@@ -395,6 +695,7 @@ struct scc_batch_plan {
     int32_t* d_live2 = nullptr;
     int32_t* d_ctr = nullptr;
     int32_t* h_ctr = nullptr;
+    int32_t max_n = 0;          // vertices of the largest graph
     scc_batch_tuning tune;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -416,8 +717,17 @@ static int batch_enqueue(scc_batch_plan* p, int sms) {
     a.ctr = p->d_ctr;
     a.warp_deg = p->tune.warp_deg;
     a.members = nullptr;
+    // Marks of the largest graph, up to 200 KB (204,800 vertices); larger graphs
+    // take the rounds over global marks from the start.  Where the marks leave
+    // fewer blocks resident than asked for, the others follow: no block waits
+    // for another.
+    const int32_t smem = std::min(200 * 1024, (p->max_n + 3) & ~3);
+    a.marks_cap = smem;
+    a.vec_adj = ((reinterpret_cast<uintptr_t>(g->node_idx) | reinterpret_cast<uintptr_t>(g->r_node_idx)) & 15u) == 0;
+    a.adj_len = g->m;
+    SCC_CUDA(cudaFuncSetAttribute(k_batch_scc, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     SCC_CUDA(cudaMemsetAsync(p->d_ctr, 0, sizeof(int32_t) * BATCH_CTR_WORDS, s->stream));
-    k_batch_scc<<<sms * p->tune.blocks_per_sm, p->tune.threads, 0, s->stream>>>(a);
+    k_batch_scc<<<sms * p->tune.blocks_per_sm, p->tune.threads, smem, s->stream>>>(a);
     SCC_CUDA(cudaPeekAtLastError());
     SCC_CUDA(cudaMemcpyAsync(p->h_ctr, p->d_ctr, sizeof(int32_t) * BATCH_CTR_WORDS, cudaMemcpyDeviceToHost,
                              s->stream));
@@ -459,6 +769,7 @@ extern "C" int scc_batch_plan_create(const scc_graph* g, scc_state* s, const int
     SCC_CUDA(cudaSetDevice(s->device));
     scc_batch_plan* p = new scc_batch_plan();
     p->g = g; p->s = s; p->G = num_graphs;
+    for (int32_t i = 0; i < num_graphs; ++i) p->max_n = std::max(p->max_n, offsets[i + 1] - offsets[i]);
     if (tuning) p->tune = *tuning; else scc_batch_default_tuning(&p->tune);
     if (!batch_tuning_ok(&p->tune)) { delete p; scc_set_error("bad batch tuning"); return SCC_ERR_INVALID; }
     cudaEventCreate(&p->ev[0]); cudaEventCreate(&p->ev[1]);
@@ -649,6 +960,9 @@ int scc_impl_resolve_tail(const scc_graph* g, scc_state* s, bool* taken) {
     a.ctr = ctr;
     a.warp_deg = 32;
     a.members = members;
+    a.marks_cap = 0;
+    a.vec_adj = 0;
+    a.adj_len = g->m;
     int sms = 148;
     SCC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
     k_batch_scc<<<sms * 2, 512, 0, st>>>(a);
