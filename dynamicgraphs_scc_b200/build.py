@@ -28,6 +28,7 @@ CU_SOURCES = [
     "scc_fb.cu",
     "scc_reach.cu",
     "scc_tile.cu",
+    "scc_record.cu",
     "scc_batch.cu",
     "scc_wcc.cu",
     "scc_run.cu",

@@ -32,6 +32,7 @@
 #include <algorithm>
 #include "scc_round.cuh"
 #include "scc_tile.cuh"
+#include "scc_record.cuh"
 
 // switch points come from the state's tunables (scc_tuning)
 #define ASYNC_EMPTY (-1)
@@ -803,6 +804,14 @@ int scc_impl_reach(const scc_graph* g, scc_state* s, RoundArgs& a, int32_t qlen)
     // kernels expand it over the whole grid
     int narrow = ((int64_t)a.live_count <= 4LL * s->tune.async_max && s->h_ctr[CTR_MAXDEG] <= a.huge_deg)
                      ? s->tune.async_after : 0;
+    const int32_t maxdeg = s->h_ctr[CTR_MAXDEG];
+    int64_t reached = qlen;                 // items (vertices x directions) of all frontiers so far
+    RecordSet records;
+    // The record drain also takes a frontier of up to four times the plain
+    // drain's, once it falls: its warps still keep up with that many items, and
+    // each level it replaces is a launch and a host round trip (the second
+    // round of a 2501 x 2501 grid: 16 levels of 30-50 us from 140,000 items on).
+    bool falling = false;
     bool bottom_up = false;
     double t0 = scc_trace_on() ? now_ms() : 0.0;
     int32_t live_lo = -1, live_hi = -1;     // live id range, read once when the tile drain is considered
@@ -826,6 +835,24 @@ int scc_impl_reach(const scc_graph* g, scc_state* s, RoundArgs& a, int32_t qlen)
             narrow = 0;
             bottom_up = false;
             if (scc_trace_on()) fprintf(stderr, "[scc] reach tile handed back %d items\n", qlen);
+            continue;
+        } else if ((falling || (qlen <= s->tune.async_max && narrow >= s->tune.async_after)) &&
+                   scc_impl_records_pay(s, a, records, live2 - reached, live_edges, maxdeg)) {
+            // narrow (or falling) frontier of a sparse round with far to go: the record drain
+            int32_t handed = 0;
+            SCC_TRY(scc_impl_reach_records(s, a, records, qin, qlen, qout, &handed));
+            if (records.unusable) continue;      // no scratch: the plain drain takes the frontier
+            if (scc_trace_on()) {
+                double t1 = now_ms();
+                fprintf(stderr, "[scc] reach records %.3f ms\n", t1 - t0);
+                t0 = t1;
+            }
+            if (handed == 0) return SCC_OK;
+            qlen = handed;
+            int32_t* t = qin; qin = qout; qout = t;
+            narrow = 0;
+            bottom_up = false;
+            falling = false;
             continue;
         } else if (qlen <= s->tune.async_max && narrow >= s->tune.async_after) {
             int64_t qcap = 2LL * s->n + 64;
@@ -946,6 +973,10 @@ int scc_impl_reach(const scc_graph* g, scc_state* s, RoundArgs& a, int32_t qlen)
             t0 = t1;
         }
         narrow = (!bottom_up && next <= s->tune.async_max && edges_small) ? narrow + 1 : 0;
+        falling = next < qlen && next <= 4 * s->tune.async_max && maxdeg <= a.huge_deg;
+        reached += next;
+        if (falling && bottom_up && scc_impl_records_pay(s, a, records, live2 - reached, live_edges, maxdeg))
+            bottom_up = false;
         qlen = next;
         int32_t* t = qin; qin = qout; qout = t;
     }

@@ -1,0 +1,28 @@
+// Record drain (scc_record.cu): interface for the traversal driver in scc_reach.cu.
+#pragma once
+#include "scc_round.cuh"
+
+// One round's records, built at its first narrow frontier and kept until the
+// round's traversal ends.  Scratch comes from the library's pool on the state's
+// stream.
+struct RecordSet {
+    cudaStream_t st = nullptr;
+    int4* rec = nullptr;          // [2 x live] records, REC_W entries each
+    uint8_t* pm = nullptr;        // [live] marks by place in the live list
+    bool unusable = false;        // scratch could not be had: the round keeps to the plain drain
+    ~RecordSet() {
+        if (rec) cudaFreeAsync(rec, st);
+        if (pm) cudaFreeAsync(pm, st);
+    }
+};
+
+// Does a narrow frontier of this round go to the record drain?  left: items
+// (vertices x directions) not reached yet; live_edges, maxdeg: total and
+// largest in+out degree of the live vertices.
+bool scc_impl_records_pay(const scc_state* s, const RoundArgs& a, const RecordSet& rs, int64_t left,
+                          unsigned long long live_edges, int32_t maxdeg);
+// Drains the qlen items of qin.  On return either the traversal is complete
+// (*handed_back = 0) or its *handed_back unexpanded items are in qout.  When
+// rs.unusable comes back set, nothing was done.
+int scc_impl_reach_records(scc_state* s, RoundArgs& a, RecordSet& rs, const int32_t* qin, int32_t qlen, int32_t* qout,
+                           int32_t* handed_back);
