@@ -193,6 +193,27 @@ static RoundArgs round_args(const scc_graph* g, scc_state* s) {
     return a;
 }
 
+// The round, or what follows its pivots, in one launch; the drains finish a
+// narrow frontier that it leaves.
+static int fb_coop(const scc_graph* g, scc_state* s, RoundArgs& a, int mode, bool pipeline, int32_t* scc_found,
+                   int32_t* active, bool* taken) {
+    int32_t left = 0;
+    ReachStart start;
+    SCC_TRY(scc_impl_round_coop(g, s, a, mode, a.use_only != 0, taken, &left, &start));
+    if (!*taken) return SCC_OK;
+    if (active) *active = s->h_ctr[CTR_NUM_CLASSES];
+    if (left > 0) {
+        SCC_TRY(scc_impl_reach(g, s, a, left, &start));
+        SCC_TRY(scc_zero_counters(s, CTR_COUNT, 3));
+        k_classify<<<scc_blocks(s->live_count), SCC_THREADS, 0, s->stream>>>(a);
+        SCC_LAUNCHED(s);
+        if (!pipeline) SCC_TRY(scc_sync_counters(s));
+    }
+    // inside the pipeline the caller's compaction synchronises next
+    *scc_found = pipeline ? -1 : s->h_ctr[CTR_COUNT];
+    return SCC_OK;
+}
+
 // One FW-BW round over every live class (only_color == INT32_MIN) or one class.
 // Requires the live list.  *scc_found = vertices finished, *active = classes pivoted.
 int scc_impl_fb_round(const scc_graph* g, scc_state* s, int32_t only_color, int32_t forced_pivot,
@@ -211,6 +232,11 @@ int scc_impl_fb_round(const scc_graph* g, scc_state* s, int32_t only_color, int3
     a.use_only = (only_color != INT32_MIN);
     a.only_color = only_color;
     unsigned blocks = scc_blocks(s->live_count);
+    bool taken = false;
+    if (forced_pivot < 0 && s->pivot_mode == SCC_PIVOT_DEGREE && s->log_cap == 0) {
+        SCC_TRY(fb_coop(g, s, a, COOP_ROUND, pipeline, scc_found, active, &taken));
+        if (taken) return SCC_OK;
+    }
     SCC_TRY(scc_zero_counters(s, CTR_COUNT, 4));
     SCC_TRY(scc_zero_counters(s, CTR_NUM_CLASSES, 1));
     SCC_TRY(scc_zero_counters(s, CTR_LIVE_EDGES, 2));
@@ -241,6 +267,8 @@ int scc_impl_fb_round(const scc_graph* g, scc_state* s, int32_t only_color, int3
             SCC_LAUNCHED(s);
         }
     }
+    SCC_TRY(fb_coop(g, s, a, COOP_SEEDED, pipeline, scc_found, active, &taken));
+    if (taken) return SCC_OK;
     SCC_TRY(scc_sync_counters(s));
     if (s->h_ctr[CTR_ERROR]) SCC_TRY(scc_check_device_error(s));
     int32_t qlen = s->h_ctr[CTR_QLEN];

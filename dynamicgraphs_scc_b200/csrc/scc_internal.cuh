@@ -70,11 +70,18 @@ enum {
     CTR_ASYNC_ITEMS = 20,// u64 (slots 20-21): items expanded by the asynchronous drain (ledger)
     CTR_ASYNC_EDGES = 22,// u64 (slots 22-23): edges scanned by it
     CTR_MAXDEG = 24,     // largest in+out degree among the vertices a round traverses
+    // how a one-launch round ended
+    CTR_COOP_CODE = 25,  // 0 complete, 1 a narrow frontier is left to the drains
+    CTR_COOP_LEFT,       // its length
+    CTR_COOP_WHICH,      // the queue it is in (0: qa, 1: qb)
+    CTR_COOP_LEVELS,     // levels run
+    CTR_COOP_REACHED = 30, // i64 (slots 30-31): items of all frontiers
     // asynchronous traversal queue counters, one 128-byte line each (polled by idle warps)
     CTR_AHEAD = 32,
     CTR_ATAIL = 64,
     CTR_AWORK = 96,
-    CTR_MAX = 128
+    CTR_MAX = 128,
+    CTR_COOP_WORDS = 320 // control words of a one-launch round, behind the counters
 };
 
 // device error codes written to CTR_ERROR

@@ -411,10 +411,7 @@ __device__ __forceinline__ void probe_chunk(const RoundArgs& a, const int32_t* _
 // after the other; P = 8 (a whole 32-byte sector per probe) needs 64
 // registers, halves the resident warps and is slower on both (1.38, 2.48 ms).
 template <int P>
-__global__ void __launch_bounds__(REACH_THREADS) k_reach_bottomup(RoundArgs a, int32_t* __restrict__ qout) {
-    __shared__ int32_t sbuf[REACH_THREADS / 32][WBUF];
-    int wid = threadIdx.x >> 5;
-    GlobalPush push{sbuf[wid], 0, qout, a.ctr + CTR_QLEN, nullptr, nullptr, 0ull};
+__device__ __forceinline__ void bottomup_pass(const RoundArgs& a, GlobalPush& push) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int64_t limit = (((int64_t)a.live_count + 31) / 32) * 32;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < limit; i += stride) {
@@ -473,6 +470,284 @@ __global__ void __launch_bounds__(REACH_THREADS) k_reach_bottomup(RoundArgs a, i
         push(p1, v | (1 << DIR_SHIFT));
     }
     push.flush();
+}
+
+template <int P>
+__global__ void __launch_bounds__(REACH_THREADS) k_reach_bottomup(RoundArgs a, int32_t* __restrict__ qout) {
+    __shared__ int32_t sbuf[REACH_THREADS / 32][WBUF];
+    GlobalPush push{sbuf[threadIdx.x >> 5], 0, qout, a.ctr + CTR_QLEN, nullptr, nullptr, 0ull};
+    bottomup_pass<P>(a, push);
+}
+
+// ------------------------------------------------------------------ one-launch round
+// A whole round -- pivots of every class, the levels, the classification -- in
+// one cooperative launch, with grid barriers where the host-driven round has
+// kernel boundaries and host round trips (about 2 us against 15-30 us a
+// level).  Lists above COOP_DEG entries are cut into chunks that the next
+// half-step spreads over all blocks, hubs and mid-degree vertices alike.  The
+// sweeps run on four blocks per SM where the bottom-up kernel alone has six,
+// and still gain on the largest graphs: a decomposition of R-MAT s16 takes 0.30 ms
+// against 0.43, the hubs graph (1 M vertices, 17 M edges) 0.55 against 0.74,
+// R-MAT s24 1.54 against 1.62, C2 16.5 against 16.8.  The
+// direction rule is scc_impl_reach's.  A frontier that the drains should
+// finish ends the launch: the host continues from the queue it is left in.
+//
+// Values that other blocks wrote in this launch are read past L1 (__ldcg,
+// volatile): queues, counters, chunk lists, slots, marks.  Colours and CSR do
+// not change before the classification, which only reads its own vertices.
+#define COOP_CHUNK 1024              // entries of one chunk (at least; more on graphs of that mean degree)
+#define COOP_DEG 256                 // lists longer than this are cut into chunks
+#define COOP_NARROW 12               // narrow levels run here before the plain drain takes over
+#define COOP_WAIT_LIMIT (1 << 24)
+#define COOP_MAX_DEGREE 128          // mean degree up to which the chunk list fits its buffer
+// control words (one 128-byte line each where blocks poll or add)
+#define CC_BAR 0
+#define CC_Q 32                      // three rotating frontier lengths, a line each
+#define CC_CHUNKS 128                // three rotating chunk counts
+#define CC_EDGES 224                 // three rotating frontier edge counts (u64)
+static_assert(CC_EDGES + 96 <= CTR_COOP_WORDS, "control words");
+
+struct CoopArgs {
+    int32_t* q[2];
+    int32_t* chunk_item; long long* chunk_at;
+    int32_t chunk;
+    int32_t* cc;
+    int32_t mode;                    // COOP_ROUND, COOP_SEEDED or COOP_REACH
+    int32_t one_class;
+    int32_t bu_alpha, bu_div, async_max;
+    long long live2;
+};
+
+// Grid barrier, bounded: false, with the error word set, when some block did not arrive.
+__device__ __forceinline__ bool coop_barrier(const RoundArgs& a, int32_t* cc, int32_t& target) {
+    __syncthreads();
+    target += gridDim.x;
+    int ok = 1;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(cc + CC_BAR, 1);
+        int spins = 0;
+        while (*(volatile int32_t*)(cc + CC_BAR) < target) {
+            if (++spins > COOP_WAIT_LIMIT) {
+                ok = 0;
+                atomicExch(a.ctr + CTR_ERROR, SCC_DEVERR_WAIT_LIMIT);
+                atomicExch(a.ctr + CTR_ERROR_INFO, 4);
+                break;
+            }
+        }
+        __threadfence();
+    }
+    return __syncthreads_and(ok);
+}
+
+// Counters of a round and the control words, before the launch.  A seeded one
+// keeps its frontier length, class count and degree totals; COOP_REACH is given its totals here.
+__global__ void k_round_begin(int32_t* ctr, int32_t* cc, int32_t mode, unsigned long long live_edges) {
+    const int t = threadIdx.x;
+    for (int i = t; i < CTR_COOP_WORDS; i += blockDim.x) cc[i] = 0;
+    if (t < 3) ctr[CTR_COUNT + t] = 0;
+    if (t == 0 && mode != COOP_SEEDED) {
+        *reinterpret_cast<unsigned long long*>(ctr + CTR_LIVE_EDGES) = live_edges;
+        ctr[CTR_MAXDEG] = mode == COOP_REACH ? INT32_MAX : 0;
+    }
+    if (t == 0 && mode == COOP_ROUND) ctr[CTR_QLEN] = ctr[CTR_NUM_CLASSES] = ctr[CTR_SPARE4] = 0;
+}
+
+__global__ void __launch_bounds__(REACH_THREADS, 4) k_round_coop(RoundArgs a, CoopArgs c) {
+    __shared__ int32_t sbuf[REACH_THREADS / 32][WBUF];
+    const unsigned full = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, threads = (int64_t)gridDim.x * blockDim.x;
+    const int64_t live_limit = (((int64_t)a.live_count + 31) / 32) * 32;
+    int32_t target = 0;
+    int32_t* cc = c.cc;
+    if (c.mode == COOP_ROUND) {
+        // slots of the classes present
+        if (c.one_class) {
+            if (tid == 0) {
+                a.slot_key[a.only_color + 1] = 0ull;
+                a.slot_pivot[a.only_color + 1] = SCC_NIL_NODE;
+                a.slot_count[a.only_color + 1] = 0;
+            }
+        } else {
+            int32_t last = INT32_MIN;
+            for (int64_t i = tid; i < live_limit; i += threads) {
+                int32_t k = SCC_COLOR_DONE;
+                if (i < a.live_count) k = a.color[a.live[i]];
+                const unsigned grp = __match_any_sync(full, k);
+                if (k != SCC_COLOR_DONE && lane == __ffs(grp) - 1 && k != last) {
+                    a.slot_key[k + 1] = 0ull;
+                    a.slot_pivot[k + 1] = SCC_NIL_NODE;
+                    a.slot_count[k + 1] = 0;
+                    last = k;
+                }
+            }
+        }
+        if (!coop_barrier(a, cc, target)) return;
+        // best pivot key per class, classes listed at their first key; degree totals
+        unsigned long long deg = 0;
+        unsigned dmax = 0;
+        for (int64_t i = tid; i < live_limit; i += threads) {
+            int32_t k = SCC_COLOR_DONE;
+            unsigned long long key = 0ull;
+            if (i < a.live_count) {
+                const int32_t v = a.live[i];
+                k = a.color[v];
+                if (k == SCC_COLOR_DONE || (a.use_only && k != a.only_color)) {
+                    k = SCC_COLOR_DONE;
+                } else {
+                    const unsigned outd = (unsigned)(__ldg(a.begin + v + 1) - __ldg(a.begin + v));
+                    const unsigned ind = (unsigned)(__ldg(a.r_begin + v + 1) - __ldg(a.r_begin + v));
+                    unsigned long long prod = (unsigned long long)outd * ind;
+                    if (prod > 0xFFFFFFFEull) prod = 0xFFFFFFFEull;
+                    key = ((prod + 1ull) << 32) | pivot_hash((uint32_t)v ^ a.pivot_salt);
+                    deg += outd + ind;
+                    dmax = max(dmax, outd + ind);
+                }
+            }
+            const unsigned grp = __match_any_sync(full, k);
+            if (grp == full) {
+                for (int o = 16; o > 0; o >>= 1) {
+                    const unsigned long long other = __shfl_xor_sync(full, key, o);
+                    key = other > key ? other : key;
+                }
+            }
+            if ((grp != full || lane == 0) && k != SCC_COLOR_DONE && key > __ldcg(a.slot_key + k + 1)) {
+                if (atomicMax(a.slot_key + k + 1, key) == 0ull) c.chunk_item[atomicAdd(a.ctr + CTR_SPARE4, 1)] = k;
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            deg += __shfl_down_sync(full, deg, o);
+            dmax = max(dmax, __shfl_down_sync(full, dmax, o));
+        }
+        if (lane == 0) {
+            if (deg) atomicAdd(reinterpret_cast<unsigned long long*>(a.ctr + CTR_LIVE_EDGES), deg);
+            if (dmax) atomicMax(a.ctr + CTR_MAXDEG, (int32_t)min(dmax, 0x7FFFFFFFu));
+        }
+        if (!coop_barrier(a, cc, target)) return;
+        const int32_t nc = __ldcg(a.ctr + CTR_SPARE4);
+        for (int64_t i = tid; i < nc; i += threads) {
+            const int32_t k = __ldcg(c.chunk_item + i);
+            const uint32_t key = (uint32_t)__ldcg(a.slot_key + k + 1);
+            seed_pivot(a, (int32_t)((uint32_t)pivot_unhash(key) ^ a.pivot_salt), k, c.q[0]);
+        }
+        if (!coop_barrier(a, cc, target)) return;
+    }
+    const unsigned long long live_edges =
+        max(1ull, __ldcg(reinterpret_cast<unsigned long long*>(a.ctr + CTR_LIVE_EDGES)));
+    const bool sparse = __ldcg(a.ctr + CTR_MAXDEG) <= a.huge_deg &&
+                        live_edges <= REC_SPARSE * (unsigned long long)a.live_count;
+    int32_t n = __ldcg(a.ctr + CTR_QLEN);
+    long long reached = n;
+    int which = 0, narrow = 0, level = 0, code = 0;
+    bool bottom_up = false;
+    while (n > 0) {
+        const int32_t* qin = which ? c.q[1] : c.q[0];
+        int32_t* qout = which ? c.q[0] : c.q[1];
+        const int o = (level + 1) % 3, z = (level + 2) % 3;
+        if (tid == 0) {              // the counters of the level after next
+            cc[CC_Q + 32 * z] = 0;
+            cc[CC_CHUNKS + 32 * z] = 0;
+            *reinterpret_cast<unsigned long long*>(cc + CC_EDGES + 32 * z) = 0ull;
+        }
+        unsigned long long* edges = reinterpret_cast<unsigned long long*>(cc + CC_EDGES + 32 * o);
+        if (bottom_up) {
+            GlobalPush push{sbuf[wid], 0, qout, cc + CC_Q + 32 * o, nullptr, nullptr, 0ull};
+            bottomup_pass<4>(a, push);
+        } else {
+            GlobalPush push{sbuf[wid], 0, qout, cc + CC_Q + 32 * o, a.begin, a.r_begin, 0ull};
+            // 32 items a warp, longest first through the chunk list
+            const int64_t groups = ((int64_t)n + 31) >> 5;
+            for (int64_t gi = tid >> 5; gi < groups; gi += threads >> 5) {
+                const int64_t idx = gi * 32 + lane;
+                bool valid = idx < n;
+                const int32_t it = valid ? __ldcg(qin + idx) : 0;
+                const int32_t v = it & ITEM_MASK;
+                const int32_t* off = ((it >> DIR_SHIFT) & 1) ? a.r_begin : a.begin;
+                const int32_t d = valid ? __ldg(off + v + 1) - __ldg(off + v) : 0;
+                if (d > COOP_DEG) {
+                    const int32_t m = (d + c.chunk - 1) / c.chunk;
+                    const int32_t at = atomicAdd(cc + CC_CHUNKS + 32 * o, m);
+                    for (int32_t j = 0; j < m; ++j) {
+                        c.chunk_item[at + j] = it;
+                        c.chunk_at[at + j] = (long long)j * c.chunk;
+                    }
+                    valid = false;
+                }
+                expand_warp(a, valid, it, push);
+            }
+            push.finish(edges);
+            if (!coop_barrier(a, cc, target)) return;
+            const int32_t chunks = __ldcg(cc + CC_CHUNKS + 32 * o);
+            if (chunks > 0) {
+                push.edges = 0ull;
+                for (int32_t x = blockIdx.x; x < chunks; x += gridDim.x) {
+                    const int32_t it = __ldcg(c.chunk_item + x), v = it & ITEM_MASK, dir = (it >> DIR_SHIFT) & 1;
+                    const int32_t* off = dir ? a.r_begin : a.begin;
+                    const int32_t* adj = dir ? a.r_node_idx : a.node_idx;
+                    const int32_t b = __ldg(off + v) + (int32_t)__ldcg(c.chunk_at + x);
+                    const int32_t e = min(__ldg(off + v + 1), b + c.chunk);
+                    const int32_t col = __ldg(a.color + v);
+                    for (int32_t k0 = b; k0 < e; k0 += REACH_THREADS) {
+                        const int32_t k = k0 + threadIdx.x;
+                        bool p = false;
+                        int32_t w = 0;
+                        if (k < e) { w = __ldg(adj + k); p = visit(a, w, col, dir); }
+                        push(p, w | (dir << DIR_SHIFT));
+                    }
+                }
+                push.finish(edges);
+            }
+        }
+        if (!coop_barrier(a, cc, target)) return;
+        // every block takes the same decision from the same counters
+        const int32_t next = __ldcg(cc + CC_Q + 32 * o);
+        const unsigned long long fe = __ldcg(edges);
+        bool edges_small = true;
+        if (bottom_up) {
+            bottom_up = (long long)next * c.bu_div > c.live2;
+        } else {
+            bottom_up = fe * (unsigned long long)c.bu_alpha > live_edges;
+            edges_small = fe <= (unsigned long long)a.async_bail;
+        }
+        ++level;
+        reached += next;
+        const bool pays = sparse && c.live2 - reached >= REC_MIN_LEFT;
+        const bool falling = pays && next < n && next <= 4 * c.async_max;
+        which ^= 1;
+        n = next;
+        narrow = (!bottom_up && next <= c.async_max && edges_small) ? narrow + 1 : 0;
+        if (n > 0 && (falling || (narrow > 0 && pays) || narrow >= COOP_NARROW)) { code = 1; break; }
+    }
+    if (code == 0 && c.mode != COOP_REACH) {
+        // classification, as k_classify
+        int32_t n_scc = 0, n_fw = 0, n_bw = 0;
+        for (int64_t i = tid; i < a.live_count; i += threads) {
+            const int32_t v = a.live[i];
+            const uint8_t m = __ldcg(a.mark + v);
+            if (!m) continue;
+            const int32_t k = a.color[v];
+            if ((m & 3) == 3) { a.scc[v] = __ldcg(a.slot_pivot + k + 1); a.color[v] = SCC_COLOR_DONE; n_scc++; }
+            else if (m & 1) { a.color[v] = __ldcg(a.slot_fw + k + 1); n_fw++; }
+            else { a.color[v] = __ldcg(a.slot_bw + k + 1); n_bw++; }
+            a.mark[v] = 0;
+        }
+        n_scc = (int32_t)__reduce_add_sync(full, (unsigned)n_scc);
+        n_fw = (int32_t)__reduce_add_sync(full, (unsigned)n_fw);
+        n_bw = (int32_t)__reduce_add_sync(full, (unsigned)n_bw);
+        if (lane == 0) {
+            if (n_scc) atomicAdd(a.ctr + CTR_COUNT, n_scc);
+            if (n_fw) atomicAdd(a.ctr + CTR_COUNT2, n_fw);
+            if (n_bw) atomicAdd(a.ctr + CTR_COUNT3, n_bw);
+        }
+    }
+    if (tid == 0) {
+        a.ctr[CTR_COOP_CODE] = code;
+        a.ctr[CTR_COOP_LEFT] = n;
+        a.ctr[CTR_COOP_WHICH] = which;
+        a.ctr[CTR_COOP_LEVELS] = level;
+        *reinterpret_cast<long long*>(a.ctr + CTR_COOP_REACHED) = reached;
+    }
 }
 
 // ------------------------------------------------------------------ asynchronous mode
@@ -791,9 +1066,61 @@ static bool tile_round(scc_state* s, int32_t* lo, int32_t* hi) {
 // times bu_alpha exceed the edges of the vertices being traversed; stay
 // bottom-up while the frontier holds more than 2*live/bu_div items.
 
-int scc_impl_reach(const scc_graph* g, scc_state* s, RoundArgs& a, int32_t qlen) {
-    int32_t* qin = s->qa;
-    int32_t* qout = s->qb;
+static int coop_blocks(int device, int64_t live) {
+    static int cached_sms[64] = {0}, cached_per[64] = {0};
+    int sms = 148, per = 1;
+    if (device >= 0 && device < 64 && cached_sms[device]) {
+        sms = cached_sms[device];
+        per = cached_per[device];
+    } else {
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_round_coop, REACH_THREADS, 0);
+        if (per < 1) per = 1;
+        if (device >= 0 && device < 64) { cached_per[device] = per; cached_sms[device] = sms; }
+    }
+    // a barrier costs more with more blocks: a small round takes one block an SM or fewer
+    const int64_t want = std::max<int64_t>(8, (live + 63) / 64);
+    const int64_t cap = live > (1 << 17) ? (int64_t)sms * per : sms;
+    return (int)std::min(want, cap);
+}
+
+int scc_impl_round_coop(const scc_graph* g, scc_state* s, RoundArgs& a, int mode, bool one_class, bool* taken,
+                        int32_t* left, ReachStart* start) {
+    *taken = false;
+    *left = 0;
+    if (g->m > (int64_t)COOP_MAX_DEGREE * g->n || s->tune.tile_min_live > 0) return SCC_OK;
+    CoopArgs c;
+    c.q[0] = s->qa; c.q[1] = s->qb;
+    c.chunk_item = s->hq; c.chunk_at = s->hoff;
+    c.chunk = (int32_t)std::max<int64_t>(COOP_CHUNK, 2 * g->m / std::max<int32_t>(g->n, 1) + 1);
+    c.cc = s->ctr + CTR_MAX;
+    c.mode = mode;
+    c.one_class = one_class ? 1 : 0;
+    c.bu_alpha = s->tune.bu_alpha; c.bu_div = s->tune.bu_div; c.async_max = s->tune.async_max;
+    c.live2 = 2LL * a.live_count;
+    k_round_begin<<<1, 256, 0, s->stream>>>(s->ctr, c.cc, mode, mode == COOP_REACH ? 2ull * (unsigned long long)g->m : 0ull);
+    SCC_LAUNCHED(s);
+    double t0 = scc_trace_on() ? now_ms() : 0.0;
+    void* args[2] = {&a, &c};
+    SCC_CUDA(cudaLaunchCooperativeKernel((const void*)k_round_coop, dim3(coop_blocks(s->device, a.live_count)),
+                                         dim3(REACH_THREADS), args, 0, s->stream));
+    SCC_LAUNCHED(s);
+    SCC_TRY(scc_sync_counters(s));
+    if (s->h_ctr[CTR_ERROR]) return scc_check_device_error(s);
+    *taken = true;
+    *left = s->h_ctr[CTR_COOP_CODE] ? s->h_ctr[CTR_COOP_LEFT] : 0;
+    start->which = s->h_ctr[CTR_COOP_WHICH];
+    start->reached = *reinterpret_cast<long long*>(s->h_ctr + CTR_COOP_REACHED);
+    s->traversal_steps += s->h_ctr[CTR_COOP_LEVELS];
+    if (scc_trace_on())
+        fprintf(stderr, "[scc] round in one launch: live=%d levels=%d left=%d %.3f ms\n", a.live_count,
+                s->h_ctr[CTR_COOP_LEVELS], *left, now_ms() - t0);
+    return SCC_OK;
+}
+
+int scc_impl_reach(const scc_graph* g, scc_state* s, RoundArgs& a, int32_t qlen, const ReachStart* start) {
+    int32_t* qin = start && start->which ? s->qb : s->qa;
+    int32_t* qout = start && start->which ? s->qa : s->qb;
     int64_t live2 = 2LL * (a.live_count > 0 ? a.live_count : 1);
     unsigned long long live_edges = *reinterpret_cast<unsigned long long*>(s->h_ctr + CTR_LIVE_EDGES);
     if (live_edges == 0) live_edges = 1;
@@ -805,13 +1132,14 @@ int scc_impl_reach(const scc_graph* g, scc_state* s, RoundArgs& a, int32_t qlen)
     int narrow = ((int64_t)a.live_count <= 4LL * s->tune.async_max && s->h_ctr[CTR_MAXDEG] <= a.huge_deg)
                      ? s->tune.async_after : 0;
     const int32_t maxdeg = s->h_ctr[CTR_MAXDEG];
-    int64_t reached = qlen;                 // items (vertices x directions) of all frontiers so far
+    int64_t reached = start ? start->reached : qlen;      // items (vertices x directions) of all frontiers so far
+    if (start) narrow = s->tune.async_after;              // a narrow frontier, left for the drains
     RecordSet records;
     // The record drain also takes a frontier of up to four times the plain
     // drain's, once it falls: its warps still keep up with that many items, and
     // each level it replaces is a launch and a host round trip (the second
     // round of a 2501 x 2501 grid: 16 levels of 30-50 us from 140,000 items on).
-    bool falling = false;
+    bool falling = start != nullptr;
     bool bottom_up = false;
     double t0 = scc_trace_on() ? now_ms() : 0.0;
     int32_t live_lo = -1, live_hi = -1;     // live id range, read once when the tile drain is considered

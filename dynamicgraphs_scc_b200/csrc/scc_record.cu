@@ -418,17 +418,11 @@ __global__ void __launch_bounds__(REC_THREADS, 1) k_reach_records(RoundArgs a, c
 }
 
 // ------------------------------------------------------------------ host side
-// Records cost a pass over the live vertices (2 x 64 bytes written and a few
-// gathers each), so they pay where the wave still has far to go: a sparse
-// round (a dense one ends in a few levels), no hub among its vertices (a warp
-// would walk its LONG record alone), and at least REC_MIN_LEFT items to reach.
-#define REC_SPARSE 10
-#define REC_MIN_LEFT (1 << 14)
 bool scc_impl_records_pay(const scc_state* s, const RoundArgs& a, const RecordSet& rs, int64_t left,
                           unsigned long long live_edges, int32_t maxdeg) {
     (void)s;
     return !rs.unusable && left >= REC_MIN_LEFT && maxdeg <= a.huge_deg &&
-           live_edges <= (unsigned long long)REC_SPARSE * (unsigned long long)a.live_count;
+           live_edges <= REC_SPARSE * (unsigned long long)a.live_count;
 }
 
 static int rec_blocks(int device) {

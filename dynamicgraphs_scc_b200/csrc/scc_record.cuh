@@ -2,6 +2,13 @@
 #pragma once
 #include "scc_round.cuh"
 
+// Records cost a pass over the live vertices (96 bytes written and a few gathers
+// each), so they pay where the wave still has far to go: a sparse round (a dense
+// one ends in a few levels), no hub among its vertices (a warp would walk its
+// LONG record alone), and at least REC_MIN_LEFT items to reach.
+#define REC_SPARSE 10ull
+#define REC_MIN_LEFT (1 << 14)
+
 // One round's records, built at its first narrow frontier and kept until the
 // round's traversal ends.  Scratch comes from the library's pool on the state's
 // stream.

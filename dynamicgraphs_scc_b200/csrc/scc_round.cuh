@@ -93,4 +93,21 @@ __device__ __forceinline__ bool visit(const RoundArgs& a, int32_t w, int32_t c, 
     return ((old >> sh) & bit) == 0u;
 }
 
-int scc_impl_reach(const scc_graph* g, scc_state* s, RoundArgs& a, int32_t qlen);
+// Where a traversal resumes that a one-launch round left: its queue and the items reached so far.
+struct ReachStart {
+    int32_t which = 0;
+    int64_t reached = 0;
+};
+// start: NULL = the frontier is the qlen items of qa.
+int scc_impl_reach(const scc_graph* g, scc_state* s, RoundArgs& a, int32_t qlen, const ReachStart* start = nullptr);
+// A round in one cooperative launch.  COOP_ROUND: degree pivots, traversal,
+// classification.  COOP_SEEDED: the pivots are in qa (their number in CTR_QLEN, the degree
+// totals in their counters).  COOP_REACH: a traversal of all of g from the items in
+// qa, without classification.  *taken is false, with nothing done, when the graph is too
+// dense for it.  *left > 0: a narrow frontier of that many items is left for
+// scc_impl_reach, and nothing is classified yet.
+#define COOP_ROUND 0
+#define COOP_SEEDED 1
+#define COOP_REACH 2
+int scc_impl_round_coop(const scc_graph* g, scc_state* s, RoundArgs& a, int mode, bool one_class, bool* taken,
+                        int32_t* left, ReachStart* start);

@@ -264,7 +264,7 @@ extern "C" int scc_state_create(const scc_graph* g, scc_state** out) {
     if (e == cudaSuccess) e = cudaMemset(s->aq, 0xFF, qb);
     if (e == cudaSuccess) e = cudaMalloc(&s->mark, (size_t)((n + 4) & ~3LL) + 4);
     if (e == cudaSuccess) e = cudaMalloc(&s->block_sums, sizeof(int32_t) * (size_t)tiles);
-    if (e == cudaSuccess) e = cudaMalloc(&s->ctr, sizeof(int32_t) * CTR_MAX);
+    if (e == cudaSuccess) e = cudaMalloc(&s->ctr, sizeof(int32_t) * (CTR_MAX + CTR_COOP_WORDS));
     if (e == cudaSuccess) e = cudaMallocHost(&s->h_ctr, sizeof(int32_t) * CTR_MAX);
     if (e == cudaSuccess) {
         for (int i = 0; i < 16 && e == cudaSuccess; ++i) e = cudaEventCreate(&s->ev[i]);

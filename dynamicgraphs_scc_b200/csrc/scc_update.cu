@@ -513,9 +513,15 @@ extern "C" int scc_update_batch(scc_graph* g, scc_state* s, int64_t n_ins, const
             // traversal over all vertices: the live list is every vertex
             SCC_TRY(scc_impl_compact_live(g, s, true));
             RoundArgs a = update_round_args(g, s);
-            *reinterpret_cast<unsigned long long*>(s->h_ctr + CTR_LIVE_EDGES) = 2ull * (unsigned long long)g->m;
-            s->h_ctr[CTR_MAXDEG] = INT32_MAX;      // degrees not scanned here: no shortcut to the drain
-            SCC_TRY(scc_impl_reach(g, s, a, qlen));
+            bool taken = false;
+            ReachStart start;
+            SCC_TRY(scc_impl_round_coop(g, s, a, COOP_REACH, true, &taken, &qlen, &start));
+            if (!taken) {
+                qlen = s->h_ctr[CTR_QLEN];
+                *reinterpret_cast<unsigned long long*>(s->h_ctr + CTR_LIVE_EDGES) = 2ull * (unsigned long long)g->m;
+                s->h_ctr[CTR_MAXDEG] = INT32_MAX;      // degrees not scanned here: no shortcut to the drain
+            }
+            if (qlen > 0) SCC_TRY(scc_impl_reach(g, s, a, qlen, taken ? &start : nullptr));
             SCC_TRY(scc_zero_counters(s, CTR_SPARE0, 1));
             k_upd_colour_region<<<scc_blocks(n), SCC_THREADS, 0, st>>>(n, s->mark, s->color, s->ctr + CTR_SPARE0);
             SCC_LAUNCHED(s);
