@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <initializer_list>
 #include <string>
 #include <vector>
 #include "scc_capi.h"
@@ -179,6 +180,7 @@ static inline unsigned scc_blocks(int64_t n, int threads = SCC_THREADS, int64_t 
 }
 int scc_sync_counters(scc_state* s);   // D2H copy of ctr -> h_ctr and stream sync
 int scc_zero_counters(scc_state* s, int first, int count);
+int scc_zero_list(scc_state* s, std::initializer_list<int> which);   // up to eight counters, one launch
 int scc_check_device_error(scc_state* s);
 
 // phase implementations shared between translation units

@@ -468,9 +468,8 @@ int scc_impl_reach_records(scc_state* s, RoundArgs& a, RecordSet& rs, const int3
     init[CTR_ATAIL - CTR_AHEAD] = announced;
     init[CTR_AWORK - CTR_AHEAD] = announced;
     SCC_CUDA(cudaMemcpyAsync(s->ctr + CTR_AHEAD, init, sizeof(init), cudaMemcpyHostToDevice, st));
-    SCC_TRY(scc_zero_counters(s, CTR_ASYNC_ITEMS, 4));
-    SCC_TRY(scc_zero_counters(s, CTR_ABAIL, 1));
-    SCC_TRY(scc_zero_counters(s, CTR_QLEN, 1));
+    SCC_TRY(scc_zero_list(s, {CTR_ASYNC_ITEMS, CTR_ASYNC_ITEMS + 1, CTR_ASYNC_EDGES, CTR_ASYNC_EDGES + 1, CTR_ABAIL,
+                              CTR_QLEN}));
     if (s->ledger_on) SCC_CUDA(cudaEventRecord(s->lev[0], st));
     k_reach_records<<<rec_blocks(s->device), REC_THREADS, 0, st>>>(a, rs.rec, rs.pm, place, s->aq, qcap, qout);
     SCC_LAUNCHED(s);

@@ -130,6 +130,16 @@ static int run_method(const scc_graph* g, scc_state* s, int method, scc_run_stat
     return SCC_OK;
 }
 
+// Representatives counted into CTR_SPARE0.
+static int count_roots(scc_state* s) {
+    SCC_TRY(scc_zero_counters(s, CTR_SPARE0, 1));
+    if (s->n > 0) {
+        k_count_roots<<<scc_blocks(s->n), SCC_THREADS, 0, s->stream>>>(s->n, s->scc, s->ctr + CTR_SPARE0);
+        SCC_LAUNCHED(s);
+    }
+    return SCC_OK;
+}
+
 extern "C" int scc_run(const scc_graph* g, scc_state* s, int method, int pivot_mode, scc_run_stats* stats) {
     SCC_REQUIRE(g && s, SCC_ERR_INVALID, "NULL argument");
     SCC_REQUIRE(s->n == g->n, SCC_ERR_INVALID, "state built for n=%d, graph has n=%d", s->n, g->n);
@@ -157,20 +167,21 @@ extern "C" int scc_run(const scc_graph* g, scc_state* s, int method, int pivot_m
     nvtxRangePop();
     s->pivot_mode = SCC_PIVOT_DEGREE;
     if (rc != SCC_OK) return rc;
-    SCC_CUDA(cudaStreamSynchronize(s->stream));
-    SCC_TRY(scc_check_device_error(s));
+    // the SCC count is enqueued behind the last phase, so one round trip ends the run
+    const int kernels = s->kernels;
+    SCC_TRY(count_roots(s));
+    SCC_TRY(scc_sync_counters(s));
+    if (s->h_ctr[CTR_ERROR]) SCC_TRY(scc_check_device_error(s));
     st.ms_trim1 = elapsed(s, 0, 1);
     st.ms_global_fb = elapsed(s, 1, 2);
     st.ms_trim12 = elapsed(s, 2, 3);
     st.ms_wcc = elapsed(s, 3, 4);
     st.ms_fb = elapsed(s, 4, 5);
     st.ms_total = elapsed(s, 0, 5);
-    st.kernels_launched = s->kernels - k0;
+    st.kernels_launched = kernels - k0;
     st.traversal_steps = s->traversal_steps - steps0;
     st.fb_rounds = s->fb_rounds - rounds0;
-    int32_t nscc = 0;
-    SCC_TRY(scc_count_sccs(s, &nscc));
-    st.num_sccs = nscc;
+    st.num_sccs = s->h_ctr[CTR_SPARE0];
     if (stats) *stats = st;
     return SCC_OK;
 }
@@ -178,11 +189,7 @@ extern "C" int scc_run(const scc_graph* g, scc_state* s, int method, int pivot_m
 extern "C" int scc_count_sccs(scc_state* s, int32_t* count) {
     SCC_REQUIRE(s && count, SCC_ERR_INVALID, "NULL argument");
     SCC_CUDA(cudaSetDevice(s->device));
-    SCC_TRY(scc_zero_counters(s, CTR_SPARE0, 1));
-    if (s->n > 0) {
-        k_count_roots<<<scc_blocks(s->n), SCC_THREADS, 0, s->stream>>>(s->n, s->scc, s->ctr + CTR_SPARE0);
-        SCC_LAUNCHED(s);
-    }
+    SCC_TRY(count_roots(s));
     SCC_TRY(scc_sync_counters(s));
     *count = s->h_ctr[CTR_SPARE0];
     return SCC_OK;

@@ -463,9 +463,7 @@ static int trim1_counting(const scc_graph* g, scc_state* s, int32_t* trimmed) {
     a.begin = g->begin; a.node_idx = g->node_idx; a.r_begin = g->r_begin; a.r_node_idx = g->r_node_idx;
     a.color = s->color; a.scc = s->scc; a.cnt = s->cnt;
     a.ovf = s->qa; a.ctr = s->ctr; a.hub = s->hq; a.snap = nullptr;
-    SCC_TRY(scc_zero_counters(s, CTR_COUNT, 1));
-    SCC_TRY(scc_zero_counters(s, CTR_OVERFLOW, 1));
-    SCC_TRY(scc_zero_counters(s, CTR_SPARE3, 1));
+    SCC_TRY(scc_zero_list(s, {CTR_COUNT, CTR_OVERFLOW, CTR_SPARE3}));
     SCC_TRY(count_self_loops(g, s));
     k_count_init<<<scc_blocks(n), SCC_THREADS, 0, s->stream>>>(g->begin, g->node_idx, g->r_begin, g->r_node_idx, n,
                                                                g->self_loops > 0 ? 1 : 0, s->cnt, s->color,
@@ -586,10 +584,7 @@ static int trim1_coloured(const scc_graph* g, scc_state* s, int32_t* trimmed) {
     a.ovf = s->qa; a.ctr = s->ctr; a.hub = s->hq; a.snap = s->aux;
     k_copy_list_i32<<<scc_blocks(n_items), SCC_THREADS, 0, s->stream>>>(s->live, n_items, s->color, s->aux);
     SCC_LAUNCHED(s);
-    SCC_TRY(scc_zero_counters(s, CTR_COUNT, 1));
-    SCC_TRY(scc_zero_counters(s, CTR_OVERFLOW, 1));
-    SCC_TRY(scc_zero_counters(s, CTR_SPARE3, 1));
-    SCC_TRY(scc_zero_counters(s, CTR_QLEN, 1));
+    SCC_TRY(scc_zero_list(s, {CTR_COUNT, CTR_OVERFLOW, CTR_SPARE3, CTR_QLEN}));
     k_ccount_init<<<scc_blocks(n_items, SCC_THREADS, 148 * 8), SCC_THREADS, 0, s->stream>>>(
         a, s->live, n_items, s->qb, s->ctr + CTR_QLEN);
     SCC_LAUNCHED(s);
@@ -758,8 +753,7 @@ int scc_impl_trim1(const scc_graph* g, scc_state* s, bool use_live, int32_t* tri
     a.begin = g->begin; a.node_idx = g->node_idx; a.r_begin = g->r_begin; a.r_node_idx = g->r_node_idx;
     a.color = s->color; a.scc = s->scc; a.ctr = s->ctr;
     a.ovf = s->qa;
-    SCC_TRY(scc_zero_counters(s, CTR_COUNT, 1));
-    SCC_TRY(scc_zero_counters(s, CTR_OVERFLOW, 1));
+    SCC_TRY(scc_zero_list(s, {CTR_COUNT, CTR_OVERFLOW}));
     if (fresh)
         k_trim1_fresh<<<scc_blocks(n_items, SCC_THREADS, 148 * 8), SCC_THREADS, 0, s->stream>>>(a, (int32_t)n_items);
     else
