@@ -929,7 +929,10 @@ int scc_impl_resolve_tail(const scc_graph* g, scc_state* s, bool* taken) {
     SCC_CUDA(pool.get((void**)&starts, sizeof(int32_t) * ((size_t)nl + 1)));
     k_tail_keys<<<scc_blocks(nl), SCC_THREADS, 0, st>>>(s->live, nl, s->color, keys);
     SCC_LAUNCHED(s);
-    SCC_TRY(scc_impl_sort_pairs_u32(keys, skeys, s->live, members, nl, 32, st));
+    // colours are at most the last one handed out (the host mirror is current here)
+    int bits = 1;
+    while (bits < 32 && (1LL << bits) <= (int64_t)s->h_ctr[CTR_NEXT_COLOR]) bits++;
+    SCC_TRY(scc_impl_sort_pairs_u32(keys, skeys, s->live, members, nl, bits, st));
     int64_t G = 0;
     SCC_TRY(scc_impl_segment_starts(skeys, nl, starts, &G, st));
     std::vector<int32_t> h((size_t)G + 1);

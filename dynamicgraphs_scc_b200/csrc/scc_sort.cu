@@ -239,6 +239,82 @@ __global__ void __launch_bounds__(RS_THREADS, 2) k_rs_scatter(const K* __restric
     }
 }
 
+// A sort of at most one tile: one block makes every pass, the keys in shared
+// memory between them, in place of five launches a pass (the recursion's tail sorts a few
+// hundred pairs).  Ranks as in k_rs_scatter, so it is stable too.
+template <typename K, bool VALS>
+__global__ void __launch_bounds__(RS_THREADS) k_rs_small(const K* __restrict__ kin, K* __restrict__ kout,
+                                                         const int32_t* __restrict__ vin, int32_t* __restrict__ vout,
+                                                         int32_t m, int passes) {
+    __shared__ int32_t wcnt[RS_WARPS][RS_BINS];
+    __shared__ K skey[RS_TILE];
+    __shared__ int32_t sval[VALS ? RS_TILE : 1];
+    __shared__ int32_t s_w[RS_WARPS];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int32_t seg = wid * RS_SEG;
+    for (int32_t j = threadIdx.x; j < m; j += RS_THREADS) {
+        skey[j] = kin[j];
+        if (VALS) sval[j] = vin[j];
+    }
+    __syncthreads();
+    for (int p = 0; p < passes; ++p) {
+        const int shift = 8 * p;
+        K k[RS_ITEMS];
+        int32_t v[RS_ITEMS], rank[RS_ITEMS];
+#pragma unroll
+        for (int r = 0; r < RS_ITEMS; ++r) {
+            const int32_t j = seg + r * 32 + lane;
+            k[r] = j < m ? skey[j] : (K)0;
+            v[r] = (VALS && j < m) ? sval[j] : 0;
+        }
+        for (int q = lane; q < RS_BINS; q += 32) wcnt[wid][q] = 0;
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < RS_ITEMS; ++r) {
+            if (seg + r * 32 >= m) continue;         // warp-uniform
+            const bool valid = seg + r * 32 + lane < m;
+            const int d = (int)((unsigned)(k[r] >> shift) & (RS_BINS - 1));
+            unsigned peers = __ballot_sync(0xFFFFFFFFu, valid);
+#pragma unroll
+            for (int bit = 0; bit < 8; ++bit) {
+                const unsigned x = __ballot_sync(0xFFFFFFFFu, (d >> bit) & 1);
+                peers &= ((d >> bit) & 1) ? x : ~x;
+            }
+            const int leader = __ffs(peers) - 1;
+            int32_t cur = (valid && lane == leader) ? wcnt[wid][d] : 0;
+            cur = __shfl_sync(0xFFFFFFFFu, cur, leader < 0 ? lane : leader);
+            rank[r] = cur + __popc(peers & lt);
+            if (valid && lane == leader) wcnt[wid][d] = cur + __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        {
+            int32_t c[RS_WARPS];
+            int32_t tot = 0;
+#pragma unroll
+            for (int w = 0; w < RS_WARPS; ++w) { c[w] = wcnt[w][threadIdx.x]; tot += c[w]; }
+            int32_t all = 0;
+            int32_t run = block_excl256(tot, s_w, &all);
+#pragma unroll
+            for (int w = 0; w < RS_WARPS; ++w) { wcnt[w][threadIdx.x] = run; run += c[w]; }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < RS_ITEMS; ++r) {
+            if (seg + r * 32 + lane >= m) continue;
+            const int32_t pos = wcnt[wid][(unsigned)(k[r] >> shift) & (RS_BINS - 1)] + rank[r];
+            skey[pos] = k[r];
+            if (VALS) sval[pos] = v[r];
+        }
+        __syncthreads();
+    }
+    for (int32_t j = threadIdx.x; j < m; j += RS_THREADS) {
+        kout[j] = skey[j];
+        if (VALS) vout[j] = sval[j];
+    }
+}
+
 static inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Scratch of one sort: the alternate key and value buffers, the per-(digit,
@@ -264,6 +340,17 @@ static int radix_sort(const K* keys_in, K* keys_out, const int32_t* vals_in, int
     if (passes == 0) {
         SCC_CUDA(cudaMemcpyAsync(keys_out, keys_in, sizeof(K) * (size_t)m, cudaMemcpyDeviceToDevice, st));
         if (vals) SCC_CUDA(cudaMemcpyAsync(vals_out, vals_in, sizeof(int32_t) * (size_t)m, cudaMemcpyDeviceToDevice, st));
+        return SCC_OK;
+    }
+    if (m <= RS_TILE) {
+        if constexpr (sizeof(K) == 4) {
+            if (vals)
+                k_rs_small<K, true><<<1, RS_THREADS, 0, st>>>(keys_in, keys_out, vals_in, vals_out, (int32_t)m, passes);
+            else
+                k_rs_small<K, false><<<1, RS_THREADS, 0, st>>>(keys_in, keys_out, nullptr, nullptr, (int32_t)m, passes);
+        } else
+            k_rs_small<K, false><<<1, RS_THREADS, 0, st>>>(keys_in, keys_out, nullptr, nullptr, (int32_t)m, passes);
+        SCC_CUDA(cudaPeekAtLastError());
         return SCC_OK;
     }
     const int32_t ntiles = (int32_t)((m + RS_TILE - 1) / RS_TILE);

@@ -293,11 +293,37 @@ static void release_graph_arrays(scc_graph* g, cudaStream_t st) {
     }
 }
 
+// The batch's pairs as one list to sort: list 0 inserts (src, dst), 1 inserts
+// (dst, src), 2 deletes (src, dst), 3 deletes (dst, src); key = list, row and column in
+// 2 + bits + bits bits.  One sort in place of four: a sort's passes are bound by their
+// launches at these sizes.
+__global__ void k_upd_pack(int64_t ki, const int32_t* __restrict__ is, const int32_t* __restrict__ id, int64_t kd,
+                           const int32_t* __restrict__ ds, const int32_t* __restrict__ dd, int32_t n, int bits,
+                           unsigned long long* __restrict__ keys, int* __restrict__ bad) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ki + kd; i += (int64_t)gridDim.x * blockDim.x) {
+        const bool del = i >= ki;
+        const int64_t j = del ? i - ki : i, k = del ? kd : ki, base = del ? 2 * ki : 0;
+        const int32_t x = del ? ds[j] : is[j], y = del ? dd[j] : id[j];
+        if (x < 0 || x >= n || y < 0 || y >= n) atomicExch(bad, 1);
+        const unsigned long long list = (unsigned long long)(del ? 2 : 0) << (2 * bits);
+        keys[base + j] = list | ((unsigned long long)(uint32_t)x << bits) | (uint32_t)y;
+        keys[base + k + j] = list | (1ull << (2 * bits)) | ((unsigned long long)(uint32_t)y << bits) | (uint32_t)x;
+    }
+}
+
+// Sorted keys to (row << 32 | column).
+__global__ void k_upd_unpack(int64_t k, int bits, unsigned long long* __restrict__ keys) {
+    const unsigned long long mask = (1ull << bits) - 1ull;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < k; i += (int64_t)gridDim.x * blockDim.x) {
+        const unsigned long long x = keys[i];
+        keys[i] = (((x >> bits) & mask) << 32) | (x & mask);
+    }
+}
+
 // keys (a<<32|b) sorted ascending into out (k entries); invalid ids flagged in *bad.
 static int sorted_keys(int64_t k, const int32_t* d_a, const int32_t* d_b, int32_t n, cudaStream_t st,
-                       DevBuf& out, int* d_bad) {
+                       unsigned long long* out, int* d_bad) {
     DevBuf tmpk;
-    SCC_TRY(alloc(out, sizeof(unsigned long long) * (size_t)k, st));
     SCC_TRY(alloc(tmpk, sizeof(unsigned long long) * (size_t)k, st));
     if (k == 0) return SCC_OK;
     k_upd_keys<<<scc_blocks(k), SCC_THREADS, 0, st>>>(k, d_a, d_b, n, tmpk.as<unsigned long long>(), d_bad);
@@ -305,7 +331,40 @@ static int sorted_keys(int64_t k, const int32_t* d_a, const int32_t* d_b, int32_
     // a < n in the high word: the bits above 32 + log2(n) are zero
     int hb = 1;
     while (hb < 31 && (1LL << hb) < (int64_t)n) hb++;
-    return scc_impl_sort_keys_u64(tmpk.as<unsigned long long>(), out.as<unsigned long long>(), k, 32 + hb, st);
+    return scc_impl_sort_keys_u64(tmpk.as<unsigned long long>(), out, k, 32 + hb, st);
+}
+
+// The four sorted lists (see k_upd_pack) one after another in out, and where each begins.
+struct BatchKeys {
+    DevBuf all;
+    unsigned long long *ins = nullptr, *ins_t = nullptr, *del = nullptr, *del_t = nullptr;
+};
+static int sort_batch(BatchKeys& b, int64_t ki, const int32_t* is, const int32_t* id, int64_t kd, const int32_t* ds,
+                      const int32_t* dd, int32_t n, cudaStream_t st, int* d_bad) {
+    const int64_t total = 2 * (ki + kd);
+    SCC_TRY(alloc(b.all, sizeof(unsigned long long) * (size_t)total, st));
+    b.ins = b.all.as<unsigned long long>();
+    b.ins_t = b.ins + ki;
+    b.del = b.ins_t + ki;
+    b.del_t = b.del + kd;
+    if (total == 0) return SCC_OK;
+    if (total >= (1LL << 31)) {          // beyond one sort: each list by itself
+        SCC_TRY(sorted_keys(ki, is, id, n, st, b.ins, d_bad));
+        SCC_TRY(sorted_keys(ki, id, is, n, st, b.ins_t, d_bad));
+        SCC_TRY(sorted_keys(kd, ds, dd, n, st, b.del, d_bad));
+        return sorted_keys(kd, dd, ds, n, st, b.del_t, d_bad);
+    }
+    int bits = 1;
+    while (bits < 31 && (1LL << bits) < (int64_t)n) bits++;
+    DevBuf tmpk;
+    SCC_TRY(alloc(tmpk, sizeof(unsigned long long) * (size_t)total, st));
+    k_upd_pack<<<scc_blocks(ki + kd), SCC_THREADS, 0, st>>>(ki, is, id, kd, ds, dd, n, bits,
+                                                           tmpk.as<unsigned long long>(), d_bad);
+    SCC_CUDA(cudaPeekAtLastError());
+    SCC_TRY(scc_impl_sort_keys_u64(tmpk.as<unsigned long long>(), b.ins, total, 2 * bits + 2, st));
+    k_upd_unpack<<<scc_blocks(total), SCC_THREADS, 0, st>>>(total, bits, b.ins);
+    SCC_CUDA(cudaPeekAtLastError());
+    return SCC_OK;
 }
 
 // One side of the merge: where the batch's events lie in the old arrays, then
@@ -465,19 +524,15 @@ extern "C" int scc_update_batch(scc_graph* g, scc_state* s, int64_t n_ins, const
     }
     SCC_TRY(alloc(bad, sizeof(int), st));
     SCC_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), st));
-    DevBuf ins_k, ins_t, del_k, del_t;
-    SCC_TRY(sorted_keys(n_ins, is, id, n, st, ins_k, bad.as<int>()));
-    SCC_TRY(sorted_keys(n_ins, id, is, n, st, ins_t, bad.as<int>()));
-    SCC_TRY(sorted_keys(n_del, ds, dd, n, st, del_k, bad.as<int>()));
-    SCC_TRY(sorted_keys(n_del, dd, ds, n, st, del_t, bad.as<int>()));
+    BatchKeys keys;
+    SCC_TRY(sort_batch(keys, n_ins, is, id, n_del, ds, dd, n, st, bad.as<int>()));
     int hbad = 0;
     SCC_CUDA(cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     SCC_CUDA(cudaStreamSynchronize(st));
     SCC_REQUIRE(!hbad, SCC_ERR_INVALID, "batch edge endpoint outside [0, %d)", n);
 
     // 1. CSR merge, both sides
-    SCC_TRY(merge_batch(g, del_k.as<unsigned long long>(), del_t.as<unsigned long long>(), n_del,
-                        ins_k.as<unsigned long long>(), ins_t.as<unsigned long long>(), n_ins, st));
+    SCC_TRY(merge_batch(g, keys.del, keys.del_t, n_del, keys.ins, keys.ins_t, n_ins, st));
     SCC_CUDA(cudaEventRecord(s->ev[9], st));
 
     // 2. deletions: re-decompose the SCCs that lost an internal edge
@@ -486,7 +541,7 @@ extern "C" int scc_update_batch(scc_graph* g, scc_state* s, int64_t n_ins, const
     if (n_del > 0) {
         k_upd_fill<<<scc_blocks(n), SCC_THREADS, 0, st>>>(n, flag, 0);
         SCC_LAUNCHED(s);
-        k_upd_flag_split<<<scc_blocks(n_del), SCC_THREADS, 0, st>>>(n_del, del_k.as<unsigned long long>(), s->scc, flag);
+        k_upd_flag_split<<<scc_blocks(n_del), SCC_THREADS, 0, st>>>(n_del, keys.del, s->scc, flag);
         SCC_LAUNCHED(s);
         SCC_TRY(scc_zero_counters(s, CTR_SPARE0, 1));
         k_upd_colour_flagged<<<scc_blocks(n), SCC_THREADS, 0, st>>>(n, s->scc, flag, s->color, s->ctr + CTR_SPARE0);
@@ -504,7 +559,7 @@ extern "C" int scc_update_batch(scc_graph* g, scc_state* s, int64_t n_ins, const
         SCC_LAUNCHED(s);
         SCC_CUDA(cudaMemsetAsync(s->mark, 0, (size_t)((n + 4) & ~3LL), st));
         SCC_TRY(scc_zero_counters(s, CTR_QLEN, 1));
-        k_upd_seed_region<<<scc_blocks(n_ins), SCC_THREADS, 0, st>>>(n_ins, ins_k.as<unsigned long long>(), s->scc,
+        k_upd_seed_region<<<scc_blocks(n_ins), SCC_THREADS, 0, st>>>(n_ins, keys.ins, s->scc,
                                                                      s->mark, s->qa, s->ctr + CTR_QLEN);
         SCC_LAUNCHED(s);
         SCC_TRY(scc_sync_counters(s));
@@ -568,7 +623,8 @@ extern "C" int scc_insert_idea1(scc_graph* g, scc_state* s, int64_t n_ins, const
     SCC_REQUIRE(g && s, SCC_ERR_INVALID, "NULL argument");
     SCC_CUDA(cudaSetDevice(s->device));
     cudaStream_t st = s->stream;
-    DevBuf d_s, d_d, bad, ins_k, ins_t;
+    DevBuf d_s, d_d, bad;
+    BatchKeys keys;
     SCC_TRY(alloc(d_s, sizeof(int32_t) * (size_t)n_ins, st)); SCC_TRY(alloc(d_d, sizeof(int32_t) * (size_t)n_ins, st));
     if (n_ins) {
         SCC_CUDA(cudaMemcpyAsync(d_s.p, src, sizeof(int32_t) * (size_t)n_ins, cudaMemcpyHostToDevice, st));
@@ -576,14 +632,13 @@ extern "C" int scc_insert_idea1(scc_graph* g, scc_state* s, int64_t n_ins, const
     }
     SCC_TRY(alloc(bad, sizeof(int), st));
     SCC_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), st));
-    SCC_TRY(sorted_keys(n_ins, d_s.as<int32_t>(), d_d.as<int32_t>(), g->n, st, ins_k, bad.as<int>()));
-    SCC_TRY(sorted_keys(n_ins, d_d.as<int32_t>(), d_s.as<int32_t>(), g->n, st, ins_t, bad.as<int>()));
+    SCC_TRY(sort_batch(keys, n_ins, d_s.as<int32_t>(), d_d.as<int32_t>(), 0, nullptr, nullptr, g->n, st,
+                       bad.as<int>()));
     int hbad = 0;
     SCC_CUDA(cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     SCC_CUDA(cudaStreamSynchronize(st));
     SCC_REQUIRE(!hbad, SCC_ERR_INVALID, "inserted edge endpoint outside [0, %d)", g->n);
-    SCC_TRY(merge_batch(g, nullptr, nullptr, 0, ins_k.as<unsigned long long>(), ins_t.as<unsigned long long>(), n_ins,
-                        st));
+    SCC_TRY(merge_batch(g, keys.del, keys.del_t, 0, keys.ins, keys.ins_t, n_ins, st));
     SCC_TRY(scc_state_reset(s));
     return scc_run(g, s, SCC_METHOD_GLOBAL_WCC_FB, SCC_PIVOT_DEGREE, stats);
 }
