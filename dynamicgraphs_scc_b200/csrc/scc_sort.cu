@@ -11,8 +11,8 @@
 //  2. an exclusive scan of those counts gives every (digit, tile) its first
 //     output position;
 //  3. k_rs_scatter: each warp ranks its own contiguous segment of the tile
-//     (per-warp digit counts in shared memory, lanes of one digit found by
-//     ballots inside a round); a block scan over (digit, warp) turns the
+//     (per-warp digit counts in shared memory, lanes of one digit found through a
+//     word per digit inside a round); a block scan over (digit, warp) turns the
 //     counts into slots.
 //     The tile is reordered by digit in shared memory first, then written
 //     out run by run, so the writes are coalesced.  Elements keep their
@@ -141,13 +141,16 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const K* __restrict__ ke
 // [w * RS_SEG, (w + 1) * RS_SEG), read 32 consecutive ones per round, all
 // rounds' loads issued before any is ranked.  Its lanes rank them inside the
 // warp (earlier rounds first, then earlier lanes) against per-warp digit
-// counts in shared memory; the lanes of a round that share a digit are found
-// with eight ballots, one per digit bit.  One block scan over (digit, warp)
+// counts in shared memory; the lanes of a round that share a digit set their
+// bits in the digit's word (eight ballots, one per digit bit, took four times the
+// instructions: a pass over 52 M 64-bit keys 340 us, so 290 us).  One block scan over (digit, warp)
 // then gives each warp's slot for each digit; the tile is reordered by digit
 // in shared memory and written out run by run, each digit's output position
 // read once per tile into shared memory.  Within a digit the order is rounds,
 // lanes, warps -- the input order -- so the sort is stable.  Two blocks per
-// SM (registers capped at 128): a third of the time of one block per SM.
+// SM (registers capped at 128): a third of the time of one block per SM; three
+// and four take 326 and 367 us, their more numerous open runs write more
+// partial sectors.
 #define RS_SEG (RS_TILE / RS_WARPS)
 template <typename K, bool VALS>
 __global__ void __launch_bounds__(RS_THREADS, 2) k_rs_scatter(const K* __restrict__ kin, K* __restrict__ kout,
@@ -179,25 +182,29 @@ __global__ void __launch_bounds__(RS_THREADS, 2) k_rs_scatter(const K* __restric
             v[r] = (VALS && j < cnt) ? __ldcg(vin + base + j) : 0;
         }
         const int32_t gofs = offs[(int64_t)threadIdx.x * ntiles + tile];    // digit threadIdx.x
+        // lanes of a round that share a digit meet in one word of shared memory (the
+        // tile's own key storage is not in use yet)
+        uint32_t* meet = reinterpret_cast<uint32_t*>(skey) + wid * RS_BINS;
 #pragma unroll
-        for (int q = lane; q < RS_BINS; q += 32) wcnt[wid][q] = 0;
+        for (int q = lane; q < RS_BINS; q += 32) { wcnt[wid][q] = 0; meet[q] = 0u; }
         __syncwarp();
 #pragma unroll
         for (int r = 0; r < RS_ITEMS; ++r) {
             const bool valid = seg + r * 32 + lane < cnt;
             const int d = (int)((unsigned)(k[r] >> shift) & (RS_BINS - 1));
-            unsigned peers = __ballot_sync(0xFFFFFFFFu, valid);
-#pragma unroll
-            for (int bit = 0; bit < 8; ++bit) {
-                const unsigned x = __ballot_sync(0xFFFFFFFFu, (d >> bit) & 1);
-                peers &= ((d >> bit) & 1) ? x : ~x;
-            }
-            // an invalid lane may see valid peers of digit d; it neither reads nor writes
+            if (valid) atomicOr(meet + d, 1u << lane);
+            __syncwarp();
+            const unsigned peers = valid ? *(volatile uint32_t*)(meet + d) : 0u;
+            __syncwarp();
             const int leader = __ffs(peers) - 1;
-            int32_t cur = (valid && lane == leader) ? wcnt[wid][d] : 0;
+            int32_t cur = 0;
+            if (valid && lane == leader) {
+                cur = wcnt[wid][d];
+                wcnt[wid][d] = cur + __popc(peers);
+                meet[d] = 0u;
+            }
             cur = __shfl_sync(0xFFFFFFFFu, cur, leader < 0 ? lane : leader);
             rank[r] = cur + __popc(peers & lt);
-            if (valid && lane == leader) wcnt[wid][d] = cur + __popc(peers);
             __syncwarp();
         }
         __syncthreads();
