@@ -1154,6 +1154,33 @@ __global__ void __launch_bounds__(512, 1) k_tail_scc(BatchArgs a, int32_t cap, c
     }
 }
 
+// Classes of at most TAIL_ONE_BLOCK grouped members: where each begins, their
+// number, the largest, and an order to take them in, by one block.
+#define TAIL_ONE_BLOCK 4096
+__global__ void __launch_bounds__(256) k_tail_starts(const uint32_t* __restrict__ keys, int32_t nl,
+                                                     int32_t* __restrict__ starts, int32_t* __restrict__ order,
+                                                     int32_t* __restrict__ out) {
+    __shared__ int32_t s_warp[32];
+    __shared__ int32_t s_big;
+    if (threadIdx.x == 0) s_big = 0;
+    int32_t base = 0;
+    for (int32_t i0 = 0; i0 < nl; i0 += 256) {
+        const int32_t i = i0 + threadIdx.x;
+        const int32_t first = i < nl && (i == 0 || keys[i] != keys[i - 1]);
+        int32_t tot = 0;
+        const int32_t before = b_scan(first, s_warp, &tot);
+        if (first) { starts[base + before] = i; order[base + before] = base + before; }
+        base += tot;
+    }
+    if (threadIdx.x == 0) starts[base] = nl;
+    __syncthreads();
+    int32_t big = 0;
+    for (int32_t k = threadIdx.x; k < base; k += 256) big = max(big, starts[k + 1] - starts[k]);
+    atomicMax(&s_big, big);
+    __syncthreads();
+    if (threadIdx.x == 0) { out[0] = base; out[1] = s_big; }
+}
+
 int scc_impl_resolve_tail(const scc_graph* g, scc_state* s, bool* taken) {
     *taken = false;
     const int32_t nl = s->live_count;
@@ -1178,22 +1205,33 @@ int scc_impl_resolve_tail(const scc_graph* g, scc_state* s, bool* taken) {
     while (bits < 32 && (1LL << bits) <= (int64_t)s->h_ctr[CTR_NEXT_COLOR]) bits++;
     SCC_TRY(scc_impl_sort_pairs_u32(keys, skeys, s->live, members, nl, bits, st));
     int64_t G = 0;
-    SCC_TRY(scc_impl_segment_starts(skeys, nl, starts, &G, st));
-    std::vector<int32_t> h((size_t)G + 1);
-    SCC_CUDA(cudaMemcpyAsync(h.data(), starts, sizeof(int32_t) * (size_t)G, cudaMemcpyDeviceToHost, st));
-    SCC_CUDA(cudaStreamSynchronize(st));
-    h[(size_t)G] = nl;
     int32_t biggest = 0;
-    for (int64_t k = 0; k < G; ++k) biggest = std::max(biggest, h[(size_t)k + 1] - h[(size_t)k]);
-    if (biggest > s->tune.tail_class) return SCC_OK;
-    std::vector<int32_t> ord((size_t)G);
-    for (int64_t k = 0; k < G; ++k) ord[(size_t)k] = (int32_t)k;
-    std::stable_sort(ord.begin(), ord.end(), [&](int32_t x, int32_t y) { return h[x + 1] - h[x] > h[y + 1] - h[y]; });
-    if (!s->bkey) SCC_CUDA(cudaMalloc(&s->bkey, sizeof(unsigned long long) * (3 * (size_t)std::max(s->n, 1) + 3)));
-    SCC_CUDA(pool.get((void**)&order, sizeof(int32_t) * (size_t)std::max<int64_t>(G, 1)));
     SCC_CUDA(pool.get((void**)&ctr, sizeof(int32_t) * BATCH_CTR_WORDS));
-    SCC_CUDA(cudaMemcpyAsync(starts + G, &nl, sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    SCC_CUDA(cudaMemcpyAsync(order, ord.data(), sizeof(int32_t) * (size_t)G, cudaMemcpyHostToDevice, st));
+    if (nl <= TAIL_ONE_BLOCK) {
+        SCC_CUDA(pool.get((void**)&order, sizeof(int32_t) * (size_t)nl));
+        k_tail_starts<<<1, 256, 0, st>>>(skeys, nl, starts, order, s->ctr + CTR_QLEN);     // CTR_QLEN, CTR_QLEN2
+        SCC_LAUNCHED(s);
+        SCC_TRY(scc_sync_counters(s));
+        G = s->h_ctr[CTR_QLEN];
+        biggest = s->h_ctr[CTR_QLEN2];
+        if (biggest > s->tune.tail_class) return SCC_OK;
+    } else {
+        SCC_TRY(scc_impl_segment_starts(skeys, nl, starts, &G, st));
+        std::vector<int32_t> h((size_t)G + 1);
+        SCC_CUDA(cudaMemcpyAsync(h.data(), starts, sizeof(int32_t) * (size_t)G, cudaMemcpyDeviceToHost, st));
+        SCC_CUDA(cudaStreamSynchronize(st));
+        h[(size_t)G] = nl;
+        for (int64_t k = 0; k < G; ++k) biggest = std::max(biggest, h[(size_t)k + 1] - h[(size_t)k]);
+        if (biggest > s->tune.tail_class) return SCC_OK;
+        // largest first
+        std::vector<int32_t> ord((size_t)G);
+        for (int64_t k = 0; k < G; ++k) ord[(size_t)k] = (int32_t)k;
+        std::stable_sort(ord.begin(), ord.end(), [&](int32_t x, int32_t y) { return h[x + 1] - h[x] > h[y + 1] - h[y]; });
+        SCC_CUDA(pool.get((void**)&order, sizeof(int32_t) * (size_t)std::max<int64_t>(G, 1)));
+        SCC_CUDA(cudaMemcpyAsync(starts + G, &nl, sizeof(int32_t), cudaMemcpyHostToDevice, st));
+        SCC_CUDA(cudaMemcpyAsync(order, ord.data(), sizeof(int32_t) * (size_t)G, cudaMemcpyHostToDevice, st));
+    }
+    if (!s->bkey) SCC_CUDA(cudaMalloc(&s->bkey, sizeof(unsigned long long) * (3 * (size_t)std::max(s->n, 1) + 3)));
     SCC_CUDA(cudaMemsetAsync(ctr, 0, sizeof(int32_t) * BATCH_CTR_WORDS, st));
     BatchArgs a;
     a.begin = g->begin; a.adj = g->node_idx; a.rbegin = g->r_begin; a.radj = g->r_node_idx;

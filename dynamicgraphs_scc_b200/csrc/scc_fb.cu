@@ -199,7 +199,7 @@ static int fb_coop(const scc_graph* g, scc_state* s, RoundArgs& a, int mode, boo
                    int32_t* active, bool* taken) {
     int32_t left = 0;
     ReachStart start;
-    SCC_TRY(scc_impl_round_coop(g, s, a, mode, a.use_only != 0, taken, &left, &start));
+    SCC_TRY(scc_impl_round_coop(g, s, a, mode, a.use_only != 0, pipeline, taken, &left, &start));
     if (!*taken) return SCC_OK;
     if (active) *active = s->h_ctr[CTR_NUM_CLASSES];
     if (left > 0) {

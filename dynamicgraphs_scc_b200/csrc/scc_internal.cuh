@@ -105,6 +105,7 @@ struct scc_state {
     int32_t* wcc = nullptr;          // G_WCC   [n]
     int32_t* live = nullptr;         // compact trim targets [n]
     int32_t live_count = 0;          // host mirror; -1 = not built (trim_targets.size()==0)
+    bool compact_ready = false;      // live_tmp holds the list's next compaction, CTR_QLEN2 its length (consumed at once)
     int32_t* live_tmp = nullptr;     // [n] scratch list
     int32_t* qa = nullptr;           // [2n+64] traversal queue A
     int32_t* qb = nullptr;           // [2n+64] traversal queue B
@@ -185,6 +186,9 @@ int scc_check_device_error(scc_state* s);
 
 // phase implementations shared between translation units
 int scc_impl_compact_live(const scc_graph* g, scc_state* s, bool from_all);
+// Enqueues the compaction of the live list into live_tmp behind the work before
+// it; the caller synchronises the counters and sets compact_ready.
+int scc_impl_compact_enqueue(scc_state* s);
 int scc_impl_trim1(const scc_graph* g, scc_state* s, bool use_live, int32_t* trimmed);
 int scc_impl_trim2(const scc_graph* g, scc_state* s, int32_t* trimmed);
 int scc_impl_ensure_colour_cap(scc_state* s, int64_t need);

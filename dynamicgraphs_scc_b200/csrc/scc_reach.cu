@@ -1084,8 +1084,8 @@ static int coop_blocks(int device, int64_t live) {
     return (int)std::min(want, cap);
 }
 
-int scc_impl_round_coop(const scc_graph* g, scc_state* s, RoundArgs& a, int mode, bool one_class, bool* taken,
-                        int32_t* left, ReachStart* start) {
+int scc_impl_round_coop(const scc_graph* g, scc_state* s, RoundArgs& a, int mode, bool one_class, bool compact,
+                        bool* taken, int32_t* left, ReachStart* start) {
     *taken = false;
     *left = 0;
     if (g->m > (int64_t)COOP_MAX_DEGREE * g->n || s->tune.tile_min_live > 0) return SCC_OK;
@@ -1105,9 +1105,13 @@ int scc_impl_round_coop(const scc_graph* g, scc_state* s, RoundArgs& a, int mode
     SCC_CUDA(cudaLaunchCooperativeKernel((const void*)k_round_coop, dim3(coop_blocks(s->device, a.live_count)),
                                          dim3(REACH_THREADS), args, 0, s->stream));
     SCC_LAUNCHED(s);
+    // rounds of sparse graphs mostly end in a drain, before which there is nothing to compact
+    compact = compact && s->live_count > 0 && 2ull * (unsigned long long)g->m > REC_SPARSE * (unsigned long long)g->n;
+    if (compact) SCC_TRY(scc_impl_compact_enqueue(s));
     SCC_TRY(scc_sync_counters(s));
     if (s->h_ctr[CTR_ERROR]) return scc_check_device_error(s);
     *taken = true;
+    s->compact_ready = compact && s->h_ctr[CTR_COOP_CODE] == 0;
     *left = s->h_ctr[CTR_COOP_CODE] ? s->h_ctr[CTR_COOP_LEFT] : 0;
     start->which = s->h_ctr[CTR_COOP_WHICH];
     start->reached = *reinterpret_cast<long long*>(s->h_ctr + CTR_COOP_REACHED);

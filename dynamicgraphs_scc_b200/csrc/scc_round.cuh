@@ -105,9 +105,11 @@ int scc_impl_reach(const scc_graph* g, scc_state* s, RoundArgs& a, int32_t qlen,
 // totals in their counters).  COOP_REACH: a traversal of all of g from the items in
 // qa, without classification.  *taken is false, with nothing done, when the graph is too
 // dense for it.  *left > 0: a narrow frontier of that many items is left for
-// scc_impl_reach, and nothing is classified yet.
+// scc_impl_reach, and nothing is classified yet.  compact: the caller compacts the
+// live list next; a round that is likely to complete does it behind the launch
+// and leaves compact_ready, which saves the round trip between the two.
 #define COOP_ROUND 0
 #define COOP_SEEDED 1
 #define COOP_REACH 2
-int scc_impl_round_coop(const scc_graph* g, scc_state* s, RoundArgs& a, int mode, bool one_class, bool* taken,
-                        int32_t* left, ReachStart* start);
+int scc_impl_round_coop(const scc_graph* g, scc_state* s, RoundArgs& a, int mode, bool one_class, bool compact,
+                        bool* taken, int32_t* left, ReachStart* start);

@@ -253,10 +253,9 @@ int scc_check_device_error(scc_state* s) {
     return SCC_ERR_OOM;
 }
 
-// Generic compaction into `out`; returns count through *count (synchronises).
+// Generic compaction into `out`, its length into CTR_QLEN2.
 template <int MODE>
-static int compact(scc_state* s, int64_t n_items, const int32_t* list, int32_t c, int32_t* out, int32_t* count) {
-    if (n_items <= 0) { *count = 0; return SCC_OK; }
+static int compact_enqueue(scc_state* s, int64_t n_items, const int32_t* list, int32_t c, int32_t* out) {
     const int32_t tiles = (int32_t)((n_items + CMP_TILE - 1) / CMP_TILE);
     if (tiles <= CMP_ONE_WAVE) {
         SCC_CUDA(cudaMemsetAsync(s->block_sums, 0, sizeof(int32_t) * ((size_t)tiles + 1), s->stream));
@@ -273,16 +272,35 @@ static int compact(scc_state* s, int64_t n_items, const int32_t* list, int32_t c
                                                                               out);
         SCC_LAUNCHED(s);
     }
+    return SCC_OK;
+}
+
+// The same with the length through *count (synchronises).
+template <int MODE>
+static int compact(scc_state* s, int64_t n_items, const int32_t* list, int32_t c, int32_t* out, int32_t* count) {
+    if (n_items <= 0) { *count = 0; return SCC_OK; }
+    SCC_TRY(compact_enqueue<MODE>(s, n_items, list, c, out));
     SCC_TRY(scc_sync_counters(s));
     if (s->h_ctr[CTR_ERROR]) return scc_check_device_error(s);
     *count = s->h_ctr[CTR_QLEN2];
     return SCC_OK;
 }
 
+int scc_impl_compact_enqueue(scc_state* s) {
+    return compact_enqueue<CMP_LIST_LIVE>(s, s->live_count, s->live, 0, s->live_tmp);
+}
+
 // create_trim1_compact (scc_trim1.cc:266-275): from all vertices when no list
 // exists yet (create_trim1_compact_1), else from the current list (_1b).
 int scc_impl_compact_live(const scc_graph* g, scc_state* s, bool from_all) {
     int32_t cnt = 0;
+    if (s->compact_ready && !from_all && s->live_count > 0) {
+        s->compact_ready = false;
+        std::swap(s->live, s->live_tmp);
+        s->live_count = s->h_ctr[CTR_QLEN2];
+        return SCC_OK;
+    }
+    s->compact_ready = false;
     if (from_all || s->live_count < 0) {
         SCC_TRY(compact<CMP_ALL_LIVE>(s, g->n, nullptr, 0, s->live, &cnt));
     } else {

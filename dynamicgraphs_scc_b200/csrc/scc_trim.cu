@@ -200,7 +200,8 @@ __device__ __forceinline__ int32_t self_run(const int32_t* __restrict__ off, con
 __global__ void k_count_init(const int32_t* __restrict__ begin, const int32_t* __restrict__ node_idx,
                              const int32_t* __restrict__ r_begin, const int32_t* __restrict__ r_node_idx, int32_t n,
                              int has_self, unsigned long long* __restrict__ cnt, int32_t* __restrict__ color,
-                             int prefinished) {
+                             int prefinished, int32_t* __restrict__ ctr) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctr[CTR_COUNT] = ctr[CTR_OVERFLOW] = ctr[CTR_SPARE3] = 0;   // the peel's
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         int32_t v = (int32_t)i;
         if (prefinished && color[v] == SCC_COLOR_DONE) {
@@ -463,11 +464,10 @@ static int trim1_counting(const scc_graph* g, scc_state* s, int32_t* trimmed) {
     a.begin = g->begin; a.node_idx = g->node_idx; a.r_begin = g->r_begin; a.r_node_idx = g->r_node_idx;
     a.color = s->color; a.scc = s->scc; a.cnt = s->cnt;
     a.ovf = s->qa; a.ctr = s->ctr; a.hub = s->hq; a.snap = nullptr;
-    SCC_TRY(scc_zero_list(s, {CTR_COUNT, CTR_OVERFLOW, CTR_SPARE3}));
     SCC_TRY(count_self_loops(g, s));
     k_count_init<<<scc_blocks(n), SCC_THREADS, 0, s->stream>>>(g->begin, g->node_idx, g->r_begin, g->r_node_idx, n,
                                                                g->self_loops > 0 ? 1 : 0, s->cnt, s->color,
-                                                               s->prefinished ? 1 : 0);
+                                                               s->prefinished ? 1 : 0, s->ctr);
     SCC_LAUNCHED(s);
     k_count_peel<false><<<scc_blocks(n, SCC_THREADS, 148 * 8), SCC_THREADS, 0, s->stream>>>(a, n, nullptr, 0);
     SCC_LAUNCHED(s);

@@ -570,7 +570,7 @@ extern "C" int scc_update_batch(scc_graph* g, scc_state* s, int64_t n_ins, const
             RoundArgs a = update_round_args(g, s);
             bool taken = false;
             ReachStart start;
-            SCC_TRY(scc_impl_round_coop(g, s, a, COOP_REACH, true, &taken, &qlen, &start));
+            SCC_TRY(scc_impl_round_coop(g, s, a, COOP_REACH, true, false, &taken, &qlen, &start));
             if (!taken) {
                 qlen = s->h_ctr[CTR_QLEN];
                 *reinterpret_cast<unsigned long long*>(s->h_ctr + CTR_LIVE_EDGES) = 2ull * (unsigned long long)g->m;
