@@ -202,7 +202,7 @@ static int build_arrays(scc_graph* g, int64_t m, const int32_t* d_src, const int
     const size_t nb = sizeof(int32_t) * ((size_t)n + 1), mb = sizeof(int32_t) * (size_t)(mk > 0 ? mk : 1);
     // from the library's pool, as an update's arrays: four cudaMalloc calls and, at the
         // end of a graph, four cudaFree took 3.6 ms around 52 M edges and 2.2 ms around 0.3 M
-    g->async_arrays = true;
+    g->async_arrays = g->built_arrays = true;
     SCC_CUDA(scc_impl_malloc_async((void**)&g->begin, nb, st));
     SCC_CUDA(scc_impl_malloc_async((void**)&g->node_idx, mb, st));
     SCC_CUDA(scc_impl_malloc_async((void**)&g->r_begin, nb, st));
@@ -544,6 +544,9 @@ extern "C" int scc_graph_free(scc_graph* g) {
     if (!g) return SCC_OK;
     cudaSetDevice(g->device);
     if (g->owns) {
+        // cudaFree waits for the device only for memory of cudaMalloc; memory of the
+        // pool could be handed out again while another stream still reads it
+        if (g->async_arrays) cudaDeviceSynchronize();
         cudaFree(g->begin); cudaFree(g->node_idx); cudaFree(g->r_begin); cudaFree(g->r_node_idx);
     }
     delete g;

@@ -44,7 +44,8 @@ struct scc_graph {
     int32_t* r_begin = nullptr;   // [n+1]  in-CSR offsets       (gm_graph::r_begin)
     int32_t* r_node_idx = nullptr;// [m]    in-neighbours        (gm_graph::r_node_idx)
     bool owns = true;
-    bool async_arrays = false;    // arrays come from cudaMallocAsync (after an update)
+    bool async_arrays = false;    // arrays come from the library's pool (built from edges, or after an update)
+    bool built_arrays = false;    // the build's own arrays: callers on any stream may hold their pointers
     mutable int64_t self_loops = -1;  // edges u->u in the CSR; -1 = not counted yet
 };
 

@@ -352,6 +352,7 @@ extern "C" int scc_state_reset(scc_state* s) {
     SCC_LAUNCHED(s);
     SCC_CUDA(cudaStreamSynchronize(s->stream));
     s->live_count = -1;
+    s->compact_ready = false;
     s->fresh = true;
     s->prefinished = false;
     s->cnt_valid = false;

@@ -286,6 +286,10 @@ static int alloc(DevBuf& b, size_t bytes, cudaStream_t st) {
 // Replace a graph's arrays with stream-ordered ones.
 static void release_graph_arrays(scc_graph* g, cudaStream_t st) {
     int32_t* arr[4] = {g->begin, g->node_idx, g->r_begin, g->r_node_idx};
+    // the first update of a built graph waits for the device, as cudaFree does where
+    // its arrays come from cudaMalloc
+    if (g->built_arrays) cudaDeviceSynchronize();
+    g->built_arrays = false;
     for (int i = 0; i < 4; ++i) {
         if (!arr[i]) continue;
         if (g->async_arrays) cudaFreeAsync(arr[i], st);
