@@ -24,7 +24,7 @@
 // grid's wave about two hops, a chain's by eight.
 //
 // C2's wave (the 4096 x 4096 grid's giant class, 13.1 M live vertices): 18.7 ms
-// in the plain drain; 1.0 ms of building and 4.3 ms here.  2501 x 2501 grid:
+// in the plain drain; 1.0 ms of building and 4.2 ms here.  2501 x 2501 grid:
 // 10.9 ms against 0.4 + 2.4 ms.  Both waves are bound by the latency of an
 // iteration (about 1 us: one round trip and the instructions around it on two
 // warps per scheduler; one warp per scheduler 6.8 ms on C2, four no faster).
@@ -120,9 +120,9 @@ __global__ void __launch_bounds__(SCC_THREADS) k_rec_neighbours(RoundArgs a, con
 // Records grown from the neighbour lists, breadth first, as far as REC_W
 // entries go; an entry may come twice, which costs its place and a claim that
 // fails.  Bound by instruction issue (divergent lanes).  C2's grid, 13.1 M
-// vertices: 0.60 ms, and the drain after it 4.35 ms; with each entry looked up
-// among the others first, 1.45 ms and 4.07 ms, or branch-free in registers 0.94
-// and 4.11 ms.
+// vertices: 0.60 ms, and the drain after it 4.2 ms; with each entry looked up
+// among the others first, 1.45 ms and 0.3 ms less in the drain, or branch-free in
+// registers 0.94 ms and 0.25 ms less.
 __global__ void __launch_bounds__(SCC_THREADS) k_rec_grow(int32_t live_count, const int4* __restrict__ nbr,
                                                           int4* __restrict__ rec) {
     __shared__ int32_t s[REC_W][SCC_THREADS];
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(REC_THREADS, 1) k_reach_records(RoundArgs a, c
     uint32_t iter = 0;
     int32_t last_work = -1;
     uint32_t my_items = 0;                            // uniform; the ledger's totals
-    unsigned long long my_edges = 0;
+    uint32_t my_edges = 0;                            // this lane's
     while (true) {
         if (list.count == 0 && ticket == 0) {
             int32_t at = 0;
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(REC_THREADS, 1) k_reach_records(RoundArgs a, c
             ticket = (1u << REC_ITEMS) - 1u;
         }
         int32_t came = -1;
-        if ((ticket >> lane) & 1u) came = (int64_t)ticket_at + lane < qcap ? rec_ld(q + ticket_at + lane) : -1;
+        if (((ticket >> lane) & 1u) && (int64_t)ticket_at + lane < qcap) came = rec_ld(q + ticket_at + lane);
         // expand
         const int32_t k = min(REC_ITEMS, list.count), first = list.count - k;
         const int32_t ent = g < k ? reinterpret_cast<const int32_t*>(list.buf)[(first + g) * REC_W + (lane & (REC_W - 1))]
@@ -286,12 +286,16 @@ __global__ void __launch_bounds__(REC_THREADS, 1) k_reach_records(RoundArgs a, c
             r0 = __ldg(at);
             r1 = __ldg(at + 1);
         }
-        const int32_t long_id = ent == REC_LONG ? list.id[first + g] : 0;
         unsigned longs = __ballot_sync(full, ent == REC_LONG);
+        int32_t long_id = 0;
+        if (longs) {
+            if (ent == REC_LONG) long_id = list.id[first + g];
+            __syncwarp();
+        }
         list.count = first;
         net -= k;
         my_items += k;
-        my_edges += __popc(__ballot_sync(full, ent >= 0));
+        my_edges += ent >= 0;
         // hand over what the last iteration prepared
         if (give) {
             // both answers are here: the count is published before the items are
@@ -314,7 +318,7 @@ __global__ void __launch_bounds__(REC_THREADS, 1) k_reach_records(RoundArgs a, c
             const int32_t* off = ldir ? a.r_begin : a.begin;
             const int32_t* adj = ldir ? a.r_node_idx : a.node_idx;
             const int32_t b = __ldg(off + v), e = __ldg(off + v + 1);
-            my_edges += e - b;
+            if (lane == 0) my_edges += (uint32_t)(e - b);
             for (int32_t k0 = b; k0 < e; k0 += 32) {
                 const int32_t w = k0 + lane < e ? __ldg(adj + k0 + lane) : v;
                 const bool mine = w != v && __ldg(a.color + w) == c;
@@ -411,9 +415,11 @@ __global__ void __launch_bounds__(REC_THREADS, 1) k_reach_records(RoundArgs a, c
         }
         if ((iter & 7) == 0 && lane == 0) stop = rec_ld(bail);
     }
+    unsigned long long edges = my_edges;
+    for (int o = 16; o > 0; o >>= 1) edges += __shfl_down_sync(full, edges, o);
     if (lane == 0) {
         atomicAdd(reinterpret_cast<unsigned long long*>(a.ctr + CTR_ASYNC_ITEMS), (unsigned long long)my_items);
-        atomicAdd(reinterpret_cast<unsigned long long*>(a.ctr + CTR_ASYNC_EDGES), my_edges);
+        atomicAdd(reinterpret_cast<unsigned long long*>(a.ctr + CTR_ASYNC_EDGES), edges);
     }
 }
 
