@@ -68,3 +68,18 @@ def test_small_and_narrow(gpu, n):
     decompose(n, *random_graph(n, 3 * n, n))
     nn, s, d, _ = seeded_graph(rmat_scale=8, edge_factor=6, grid_side=16, seed=n)
     decompose(nn, s, d)
+
+
+@pytest.mark.parametrize("k", [8 * 1024, 8 * 1024 + 1, 9 * 1024 - 1, 600000])
+@pytest.mark.parametrize("back", [0, 1, 2])
+def test_hub_lists(gpu, k, back):
+    # a cycle of 19 with a hub of k out- and k in-neighbours, lists that a lane or its
+    # warp enters into the chunk list.  back 0: the neighbours peel off and the 19 stay live;
+    # 1: every out-neighbour returns through the cycle; 2: half of them do
+    c = np.arange(19)
+    out, inn = 19 + np.arange(k), 19 + k + np.arange(k)
+    s = np.concatenate([c, np.zeros(k, np.int64), inn])
+    d = np.concatenate([(c + 1) % 19, out, np.zeros(k, np.int64)])
+    if back:
+        s, d = np.concatenate([s, out[::back]]), np.concatenate([d, out[::back] % 19])
+    decompose(19 + 2 * k, s, d)
