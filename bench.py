@@ -67,13 +67,13 @@ WORKLOAD_NAMES = {
 }
 
 
-# DRAM traffic of the asynchronous drain relative to its algorithmic bytes,
-# from one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum over all
-# launches) of `bench.py --workload grid4096 --steps 1 --warmup 0`: 595.40 MB
-# read + written by 9 launches whose algorithmic bytes total 793.8 MB.  The
+# DRAM traffic of the record drain relative to its algorithmic bytes, from one
+# ncu capture (dram__bytes_read.sum + dram__bytes_write.sum over all launches)
+# of `bench.py --workload grid4096 --steps 1 --warmup 0`: 965.55 MB read +
+# written by 4 launches whose algorithmic bytes total 1,014.27 MB.  The
 # full C2 step is too large for that capture; its drain runs the same grid.
-ASYNC_TRAFFIC_RATIO = 595.40 / 793.8
-ASYNC_TRAFFIC_SOURCE = "ncu dram bytes on the 4096x4096 grid workload (0.750 x algorithmic), scaled per launch"
+ASYNC_TRAFFIC_RATIO = 965.55 / 1014.27
+ASYNC_TRAFFIC_SOURCE = "ncu dram bytes on the 4096x4096 grid workload (0.952 x algorithmic), scaled per launch"
 
 
 def measured_peak_gbs():
@@ -934,15 +934,15 @@ def main():
     peak, peak_kind = measured_peak_gbs()
     b_alg = 16 * m + 20 * n + 8
     achieved = b_alg / (ms * 1e-3) / 1e9
-    # dominant kernel: the asynchronous reachability drain.  Algorithmic bytes:
-    # 13 B per expanded item (offset pair, colour, mark) + 9 B per scanned edge
+    # dominant kernel: the record drain (the plain drain's launches count with
+    # it where a round takes that one).  Algorithmic bytes: 13 B per expanded item (offset pair, colour, mark) + 9 B per scanned edge
     # (neighbour id, its colour, its mark).
     kernel_roofline = None
     if l_launch.value > 0 and l_ms.value > 0:
         k_bytes = (13 * l_items.value + 9 * l_edges.value) / l_launch.value
         k_ms = l_ms.value / l_launch.value
         k_ach = k_bytes / (k_ms * 1e-3) / 1e9
-        kernel_roofline = {"bound": "hbm", "kernel": "k_reach_async", "achieved": round(k_ach, 2), "peak": peak,
+        kernel_roofline = {"bound": "hbm", "kernel": "k_reach_records", "achieved": round(k_ach, 2), "peak": peak,
                            "peak_kind": peak_kind, "unit": "GB/s", "frac": round(k_ach / peak, 5),
                            "traffic": int(ASYNC_TRAFFIC_RATIO * k_bytes), "traffic_source": ASYNC_TRAFFIC_SOURCE,
                            "bytes_per_launch": int(k_bytes), "ms_per_launch": round(k_ms, 4),

@@ -58,9 +58,10 @@ const char* scc_status_string(int status);
 const char* scc_last_error(void);
 int scc_version(void);                       /* major*10000 + minor*100 + patch */
 int scc_device_count(int* count);
-/* Scratch of uploads, updates and graph merges comes from one memory pool per
- * device owned by this library, which keeps freed blocks for reuse; this hands
- * them back to the driver (after synchronising the device). */
+/* Scratch of uploads, updates and graph merges, and the arrays of a graph built
+ * from edges, come from one memory pool per device owned by this library, which
+ * keeps freed blocks for reuse; this hands them back to the driver (after
+ * synchronising the device). */
 int scc_release_cached_memory(int device);
 /* Host-side fault injection for failure-path tests (the reference's only
  * failure path is CUDA_CHECK -> exit(1), src_CUDA/scc_cuda.h:61-67).
