@@ -1212,7 +1212,7 @@ int scc_impl_reach(const scc_graph* g, scc_state* s, RoundArgs& a, int32_t qlen,
             if (scc_trace_on()) fprintf(stderr, "[scc] reach tile handed back %d items\n", qlen);
             continue;
         } else if ((falling || (qlen <= s->tune.async_max && narrow >= s->tune.async_after)) &&
-                   scc_impl_records_pay(s, a, records, live2 - reached, live_edges, maxdeg)) {
+                   scc_impl_records_pay(a, records, live2 - reached, live_edges, maxdeg)) {
             // narrow (or falling) frontier of a sparse round with far to go: the record drain
             int32_t handed = 0;
             SCC_TRY(scc_impl_reach_records(s, a, records, qin, qlen, qout, &handed));
@@ -1350,7 +1350,7 @@ int scc_impl_reach(const scc_graph* g, scc_state* s, RoundArgs& a, int32_t qlen,
         narrow = (!bottom_up && next <= s->tune.async_max && edges_small) ? narrow + 1 : 0;
         falling = next < qlen && next <= 4 * s->tune.async_max && maxdeg <= a.huge_deg;
         reached += next;
-        if (falling && bottom_up && scc_impl_records_pay(s, a, records, live2 - reached, live_edges, maxdeg))
+        if (falling && bottom_up && scc_impl_records_pay(a, records, live2 - reached, live_edges, maxdeg))
             bottom_up = false;
         qlen = next;
         int32_t* t = qin; qin = qout; qout = t;

@@ -159,11 +159,32 @@ __global__ void __launch_bounds__(SCC_THREADS) k_rec_grow(int32_t live_count, co
     }
 }
 
-// Frontier items (vertex | direction << DIR_SHIFT) to places, and back.
-__global__ void k_rec_items_in(const int32_t* __restrict__ q, int32_t n, const int32_t* __restrict__ place,
-                               int32_t* __restrict__ out) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = place[q[i] & ITEM_MASK] | (((q[i] >> DIR_SHIFT) & 1) << REC_DIR);
+// Frontier items (vertex | direction << DIR_SHIFT) to places, and back.  Of the
+// n items of q, those of listed vertices are appended to out (count *listed, and the
+// drain's *work with it); a class vertex that the live list does not hold has no
+// place -- whatever is read for it is some earlier use's -- and goes to the host's next frontier.
+__global__ void k_rec_items_in(const int32_t* __restrict__ q, int32_t n, const int32_t* __restrict__ live,
+                               int32_t live_count, const int32_t* __restrict__ place, int32_t* __restrict__ out,
+                               int32_t* __restrict__ listed, int32_t* __restrict__ work,
+                               int32_t* __restrict__ outside, int32_t* __restrict__ outside_count) {
+    const int lane = threadIdx.x & 31;
+    const unsigned full = 0xFFFFFFFFu, lt = (1u << lane) - 1u;
+    const int64_t limit = ((int64_t)n + 31) / 32 * 32;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < limit; i += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t it = i < n ? q[i] : 0, v = it & ITEM_MASK;
+        const int32_t p = i < n ? place[v] : -1;
+        const bool in = (uint32_t)p < (uint32_t)live_count && live[p] == v;
+        const unsigned bin = __ballot_sync(full, in), bout = __ballot_sync(full, i < n && !in);
+        int32_t at = 0, oat = 0;
+        if (lane == 0) {
+            if (bin) { at = atomicAdd(listed, __popc(bin)); atomicAdd(work, __popc(bin)); }
+            if (bout) oat = atomicAdd(outside_count, __popc(bout));
+        }
+        at = __shfl_sync(full, at, 0);
+        oat = __shfl_sync(full, oat, 0);
+        if (in) out[at + __popc(bin & lt)] = p | (((it >> DIR_SHIFT) & 1) << REC_DIR);
+        else if (i < n) outside[oat + __popc(bout & lt)] = it;
+    }
 }
 // What a hand-back left anywhere in the queue, appended to out; the queue is kept empty between uses.
 __global__ void k_rec_items_out(int32_t* __restrict__ q, int32_t n, const int32_t* __restrict__ live,
@@ -424,10 +445,9 @@ __global__ void __launch_bounds__(REC_THREADS, 1) k_reach_records(RoundArgs a, c
 }
 
 // ------------------------------------------------------------------ host side
-bool scc_impl_records_pay(const scc_state* s, const RoundArgs& a, const RecordSet& rs, int64_t left,
-                          unsigned long long live_edges, int32_t maxdeg) {
-    (void)s;
-    return !rs.unusable && left >= REC_MIN_LEFT && maxdeg <= a.huge_deg &&
+bool scc_impl_records_pay(const RoundArgs& a, const RecordSet& rs, int64_t left, unsigned long long live_edges,
+                          int32_t maxdeg) {
+    return !rs.unusable && !rs.outside && left >= REC_MIN_LEFT && maxdeg <= a.huge_deg &&
            live_edges <= REC_SPARSE * (unsigned long long)a.live_count;
 }
 
@@ -466,16 +486,17 @@ int scc_impl_reach_records(scc_state* s, RoundArgs& a, RecordSet& rs, const int3
         SCC_LAUNCHED(s);
     }
     const int64_t qcap = 2LL * s->n + 64;
-    k_rec_items_in<<<scc_blocks(qlen), SCC_THREADS, 0, st>>>(qin, qlen, place, s->aq);
-    SCC_LAUNCHED(s);
     int32_t init[CTR_AWORK - CTR_AHEAD + 1] = {0};   // head, tail, work on separate lines
-    // an injected failure announces one item more than was written (as in the plain drain)
-    const int32_t announced = qlen + (scc_impl_take_wait_injection() ? 1 : 0);
-    init[CTR_ATAIL - CTR_AHEAD] = announced;
-    init[CTR_AWORK - CTR_AHEAD] = announced;
+    // an injected failure announces one item that is never written: slot 0 stays empty
+    const int32_t hole = scc_impl_take_wait_injection() ? 1 : 0;
+    init[CTR_ATAIL - CTR_AHEAD] = hole;
+    init[CTR_AWORK - CTR_AHEAD] = hole;
     SCC_CUDA(cudaMemcpyAsync(s->ctr + CTR_AHEAD, init, sizeof(init), cudaMemcpyHostToDevice, st));
     SCC_TRY(scc_zero_list(s, {CTR_ASYNC_ITEMS, CTR_ASYNC_ITEMS + 1, CTR_ASYNC_EDGES, CTR_ASYNC_EDGES + 1, CTR_ABAIL,
                               CTR_QLEN}));
+    k_rec_items_in<<<scc_blocks(qlen), SCC_THREADS, 0, st>>>(qin, qlen, a.live, L, place, s->aq, s->ctr + CTR_ATAIL,
+                                                            s->ctr + CTR_AWORK, qout, s->ctr + CTR_QLEN);
+    SCC_LAUNCHED(s);
     if (s->ledger_on) SCC_CUDA(cudaEventRecord(s->lev[0], st));
     k_reach_records<<<rec_blocks(s->device), REC_THREADS, 0, st>>>(a, rs.rec, rs.pm, place, s->aq, qcap, qout);
     SCC_LAUNCHED(s);
@@ -503,7 +524,9 @@ int scc_impl_reach_records(scc_state* s, RoundArgs& a, RecordSet& rs, const int3
         SCC_CUDA(cudaMemsetAsync(s->aq, 0xFF, sizeof(int32_t) * (size_t)qcap, st));
         return scc_check_device_error(s);
     }
-    int32_t items = s->h_ctr[CTR_QLEN];           // vertices outside the live list, already in qout
+    int32_t items = s->h_ctr[CTR_QLEN];           // already in qout
+    // class vertices outside the live list: the plain drain, which goes by vertex, does the rest
+    if (items > 0 && !s->h_ctr[CTR_ABAIL]) rs.outside = true;
     if (s->h_ctr[CTR_ABAIL] && s->h_ctr[CTR_ATAIL] > 0) {
         k_rec_items_out<<<scc_blocks(s->h_ctr[CTR_ATAIL]), SCC_THREADS, 0, st>>>(s->aq, s->h_ctr[CTR_ATAIL], a.live, qout,
                                                                                s->ctr + CTR_QLEN);

@@ -17,6 +17,7 @@ struct RecordSet {
     int4* rec = nullptr;          // [2 x live] records, REC_W entries each
     uint8_t* pm = nullptr;        // [live] marks by place in the live list
     bool unusable = false;        // scratch could not be had: the round keeps to the plain drain
+    bool outside = false;         // the wave met class vertices outside the live list: so does the rest of the round
     ~RecordSet() {
         if (rec) cudaFreeAsync(rec, st);
         if (pm) cudaFreeAsync(pm, st);
@@ -26,8 +27,8 @@ struct RecordSet {
 // Does a narrow frontier of this round go to the record drain?  left: items
 // (vertices x directions) not reached yet; live_edges, maxdeg: total and
 // largest in+out degree of the live vertices.
-bool scc_impl_records_pay(const scc_state* s, const RoundArgs& a, const RecordSet& rs, int64_t left,
-                          unsigned long long live_edges, int32_t maxdeg);
+bool scc_impl_records_pay(const RoundArgs& a, const RecordSet& rs, int64_t left, unsigned long long live_edges,
+                          int32_t maxdeg);
 // Drains the qlen items of qin.  On return either the traversal is complete
 // (*handed_back = 0) or its *handed_back unexpanded items are in qout.  When
 // rs.unusable comes back set, nothing was done.
