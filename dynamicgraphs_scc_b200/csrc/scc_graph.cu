@@ -718,19 +718,23 @@ static cudaError_t pool_of(int device, cudaMemPool_t* out) {
 }
 
 // Host-side fault injection (scc_debug_inject): the n-th pool allocation from
-// now fails; the next asynchronous drain gets one queue slot nobody fills.
+// now fails; the next asynchronous drain gets one queue slot nobody fills; the
+// next record drain's idle warps give up after a few polls.
 static std::atomic<int64_t> g_fail_alloc_in{0};
 static std::atomic<int> g_wait_hole{0};
+static std::atomic<int> g_idle_polls{0};
 
 extern "C" int scc_debug_inject(int what, int64_t countdown) {
     SCC_REQUIRE(countdown >= 0, SCC_ERR_INVALID, "countdown %lld", (long long)countdown);
     if (what == SCC_INJECT_ALLOC) { g_fail_alloc_in = countdown; return SCC_OK; }
     if (what == SCC_INJECT_WAIT) { g_wait_hole = countdown > 0 ? 1 : 0; return SCC_OK; }
+    if (what == SCC_INJECT_IDLE) { g_idle_polls = (int)std::min<int64_t>(countdown, 1 << 20); return SCC_OK; }
     scc_set_error("unknown injection %d", what);
     return SCC_ERR_INVALID;
 }
 
 bool scc_impl_take_wait_injection() { return g_wait_hole.exchange(0) != 0; }
+int scc_impl_take_idle_injection() { return g_idle_polls.exchange(0); }
 
 cudaError_t scc_impl_malloc_async(void** p, size_t bytes, cudaStream_t st) {
     int64_t k = g_fail_alloc_in.load();

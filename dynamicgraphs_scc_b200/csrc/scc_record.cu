@@ -260,7 +260,7 @@ __device__ __forceinline__ bool rec_claim(const int4* __restrict__ rec, uint8_t*
 __global__ void __launch_bounds__(REC_THREADS, 1) k_reach_records(RoundArgs a, const int4* __restrict__ rec, uint8_t* pm,
                                                                   const int32_t* __restrict__ place,
                                                                   int32_t* __restrict__ q, int64_t qcap,
-                                                                  int32_t* __restrict__ outside) {
+                                                                  int32_t* __restrict__ outside, int idle_limit) {
     static_assert(REC_W == 8, "a record is two int4 and eight lanes wide");
     const unsigned full = 0xFFFFFFFFu;
     __shared__ int4 s_buf[REC_WARPS][2 * REC_BUF];
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(REC_THREADS, 1) k_reach_records(RoundArgs a, c
                 if (w == 0 || e != 0 || bl != 0) break;
                 if (w != last_work) { last_work = w; idle = 1; }     // progress elsewhere resets the limit
             }
-            if (idle > REC_IDLE_LIMIT) {
+            if (idle > idle_limit) {
                 if (lane == 0) { atomicExch(err, SCC_DEVERR_WAIT_LIMIT); atomicExch(a.ctr + CTR_ERROR_INFO, 1); }
                 break;
             }
@@ -498,7 +498,9 @@ int scc_impl_reach_records(scc_state* s, RoundArgs& a, RecordSet& rs, const int3
                                                             s->ctr + CTR_AWORK, qout, s->ctr + CTR_QLEN);
     SCC_LAUNCHED(s);
     if (s->ledger_on) SCC_CUDA(cudaEventRecord(s->lev[0], st));
-    k_reach_records<<<rec_blocks(s->device), REC_THREADS, 0, st>>>(a, rs.rec, rs.pm, place, s->aq, qcap, qout);
+    const int idle_polls = scc_impl_take_idle_injection();
+    k_reach_records<<<rec_blocks(s->device), REC_THREADS, 0, st>>>(a, rs.rec, rs.pm, place, s->aq, qcap, qout,
+                                                                  idle_polls > 0 ? idle_polls : REC_IDLE_LIMIT);
     SCC_LAUNCHED(s);
     if (s->ledger_on) SCC_CUDA(cudaEventRecord(s->lev[1], st));
     k_rec_marks_out<<<scc_blocks(L), SCC_THREADS, 0, st>>>(a.live, L, rs.pm, a.mark);
@@ -513,26 +515,29 @@ int scc_impl_reach_records(scc_state* s, RoundArgs& a, RecordSet& rs, const int3
         s->ledger_items += *reinterpret_cast<long long*>(s->h_ctr + CTR_ASYNC_ITEMS);
         s->ledger_edges += *reinterpret_cast<long long*>(s->h_ctr + CTR_ASYNC_EDGES);
     }
-    if (s->h_ctr[CTR_ERROR] == SCC_DEVERR_WAIT_LIMIT && s->h_ctr[CTR_ERROR_INFO] == 1 &&
-        (s->h_ctr[CTR_AWORK] == 0 || s->h_ctr[CTR_ABAIL])) {
-        // idle warps gave up beside one warp's long chain, and the traversal is
-        // complete (or handed back) all the same: see the plain drain
+    int32_t items = s->h_ctr[CTR_QLEN];           // already in qout
+    // class vertices outside the live list: the plain drain, which goes by vertex, does the rest
+    if (items > 0 && !s->h_ctr[CTR_ABAIL]) rs.outside = true;
+    const bool gave_up = s->h_ctr[CTR_ERROR] == SCC_DEVERR_WAIT_LIMIT && s->h_ctr[CTR_ERROR_INFO] == 1;
+    if ((s->h_ctr[CTR_ABAIL] || (gave_up && s->h_ctr[CTR_AWORK] != 0)) && s->h_ctr[CTR_ATAIL] > 0) {
+        const int32_t work = s->h_ctr[CTR_AWORK], tail = (int32_t)std::min<int64_t>(s->h_ctr[CTR_ATAIL], qcap);
+        k_rec_items_out<<<scc_blocks(tail), SCC_THREADS, 0, st>>>(s->aq, tail, a.live, qout, s->ctr + CTR_QLEN);
+        SCC_LAUNCHED(s);
+        SCC_TRY(scc_sync_counters(s));
+        // Idle warps gave up beside one warp's long chain, on which the work count
+        // sits still; they held tickets, so what that warp shared afterwards
+        // lies at places that nobody reads.  If that is all the work there is, it is handed back.
+        if (!s->h_ctr[CTR_ABAIL] && s->h_ctr[CTR_QLEN] - items == work) s->h_ctr[CTR_AWORK] = 0;
+        items = s->h_ctr[CTR_QLEN];
+    }
+    if (gave_up && (s->h_ctr[CTR_AWORK] == 0 || s->h_ctr[CTR_ABAIL])) {
+        // the traversal is complete, or handed back, all the same: see the plain drain
         s->h_ctr[CTR_ERROR] = 0;
         SCC_CUDA(cudaMemsetAsync(s->ctr + CTR_ERROR, 0, sizeof(int32_t) * 2, st));
     }
     if (s->h_ctr[CTR_ERROR]) {
         SCC_CUDA(cudaMemsetAsync(s->aq, 0xFF, sizeof(int32_t) * (size_t)qcap, st));
         return scc_check_device_error(s);
-    }
-    int32_t items = s->h_ctr[CTR_QLEN];           // already in qout
-    // class vertices outside the live list: the plain drain, which goes by vertex, does the rest
-    if (items > 0 && !s->h_ctr[CTR_ABAIL]) rs.outside = true;
-    if (s->h_ctr[CTR_ABAIL] && s->h_ctr[CTR_ATAIL] > 0) {
-        k_rec_items_out<<<scc_blocks(s->h_ctr[CTR_ATAIL]), SCC_THREADS, 0, st>>>(s->aq, s->h_ctr[CTR_ATAIL], a.live, qout,
-                                                                               s->ctr + CTR_QLEN);
-        SCC_LAUNCHED(s);
-        SCC_TRY(scc_sync_counters(s));
-        items = s->h_ctr[CTR_QLEN];
     }
     *handed_back = items;
     if (scc_trace_on())

@@ -69,10 +69,14 @@ int scc_release_cached_memory(int device);
  * from now fails (SCC_ERR_OOM); 0 disarms.  SCC_INJECT_WAIT (countdown > 0):
  * the next asynchronous reachability drain is given one queue slot that is
  * never filled, so its bounded wait gives up and the call returns
- * SCC_ERR_TIMEOUT; the state is usable again after scc_state_reset.  No
+ * SCC_ERR_TIMEOUT; the state is usable again after scc_state_reset.
+ * SCC_INJECT_IDLE (countdown > 0): idle warps of the next record drain give up
+ * after countdown polls without progress, as they do after seconds beside a
+ * chain of tens of millions of hops; the call completes all the same.  No
  * injection faults, traps or hangs the GPU. */
 #define SCC_INJECT_ALLOC 1
 #define SCC_INJECT_WAIT  2
+#define SCC_INJECT_IDLE  3
 int scc_debug_inject(int what, int64_t countdown);
 
 /* ---- graph (gm_graph / GPUGraph) ---------------------------------------------------- */
