@@ -395,7 +395,7 @@ static int merge_events(MergeSide& x, int32_t kdel, int32_t kins, cudaStream_t s
     SCC_TRY(alloc(x.ins_at, sizeof(int32_t) * (size_t)kins, st));
     // one extra zero count: its exclusive prefix is the number of deleted entries
     SCC_CUDA(cudaMemsetAsync(cnt.as<int32_t>() + kdel, 0, sizeof(int32_t), st));
-    if (kdel + kins > 0) {
+    if ((int64_t)kdel + kins > 0) {          // two lists of 2^30 and more pass 2^31 together
         k_upd_events<<<scc_blocks((int64_t)kdel + kins), SCC_THREADS, 0, st>>>(
             kdel, x.del, kins, x.ins, x.off, x.adj, x.run_lo.as<int32_t>(), cnt.as<int32_t>(), x.ins_at.as<int32_t>());
         SCC_CUDA(cudaPeekAtLastError());
@@ -437,6 +437,8 @@ static int merge_write(MergeSide& x, int32_t n, int64_t m, int32_t kdel, int32_t
 // A failure leaves g as it was.
 static int merge_batch(scc_graph* g, const unsigned long long* del, const unsigned long long* del_t, int64_t kdel,
                        const unsigned long long* ins, const unsigned long long* ins_t, int64_t kins, cudaStream_t st) {
+    SCC_REQUIRE(kdel < (1LL << 31) && g->m + kins < (1LL << 31) - 1, SCC_ERR_INVALID,
+                "batch of %lld inserts and %lld deletes exceeds int32 edge ids", (long long)kins, (long long)kdel);
     MergeSide f, r;
     f.off = g->begin; f.adj = g->node_idx; f.del = del; f.ins = ins;
     r.off = g->r_begin; r.adj = g->r_node_idx; r.del = del_t; r.ins = ins_t;
@@ -625,6 +627,8 @@ extern "C" int scc_decremental_delete(scc_graph* g, scc_state* s, int64_t n_del,
 extern "C" int scc_insert_idea1(scc_graph* g, scc_state* s, int64_t n_ins, const int32_t* src, const int32_t* dst,
                                 scc_run_stats* stats) {
     SCC_REQUIRE(g && s, SCC_ERR_INVALID, "NULL argument");
+    SCC_REQUIRE(n_ins >= 0 && (n_ins == 0 || (src && dst)), SCC_ERR_INVALID, "bad batch");
+    SCC_REQUIRE(g->m + n_ins < (1LL << 31) - 1, SCC_ERR_INVALID, "edge count would exceed int32");
     SCC_CUDA(cudaSetDevice(s->device));
     cudaStream_t st = s->stream;
     DevBuf d_s, d_d, bad;
