@@ -121,6 +121,7 @@ struct scc_state {
     int32_t* tq = nullptr;           // tile drain inboxes [tq_cap], kept at -1 between uses (allocated at first use)
     int64_t tq_cap = 0;
     int32_t* tctr = nullptr;         // tile drain counters (allocated at first use)
+    int64_t drain_scratch = -1;      // bytes a record drain may take from the pool; -1 = any number (else: the plain drain)
     unsigned long long* bkey = nullptr;  // [3n] pivot key per colour of the one-launch tail (allocated at first use)
     int32_t* block_sums = nullptr;   // scan scratch
     int32_t* ctr = nullptr;          // device counters [CTR_MAX]

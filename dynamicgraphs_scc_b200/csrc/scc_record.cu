@@ -467,6 +467,11 @@ int scc_impl_reach_records(scc_state* s, RoundArgs& a, RecordSet& rs, const int3
     if (!rs.rec) {
         rs.st = st;
         void* nbr = nullptr;
+        static_assert(REC_W == 8, "scc_record_bytes");
+        if (s->drain_scratch >= 0 && scc_record_bytes(L) > s->drain_scratch) {
+            rs.unusable = true;
+            return SCC_OK;
+        }
         if (scc_impl_malloc_async((void**)&rs.rec, rec_bytes, st) != cudaSuccess ||
             scc_impl_malloc_async((void**)&rs.pm, ((size_t)L + 3) & ~(size_t)3, st) != cudaSuccess ||
             scc_impl_malloc_async(&nbr, rec_bytes / 2, st) != cudaSuccess) {

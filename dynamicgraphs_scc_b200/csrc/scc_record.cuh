@@ -29,6 +29,8 @@ struct RecordSet {
 // largest in+out degree of the live vertices.
 bool scc_impl_records_pay(const RoundArgs& a, const RecordSet& rs, int64_t left, unsigned long long live_edges,
                           int32_t maxdeg);
+// Bytes of pool scratch a round of `live` vertices takes: records, their marks and, while they are made, neighbours.
+static inline int64_t scc_record_bytes(int64_t live) { return 96 * live + ((live + 3) & ~3LL); }
 // Drains the qlen items of qin.  On return either the traversal is complete
 // (*handed_back = 0) or its *handed_back unexpanded items are in qout.  When
 // rs.unusable comes back set, nothing was done.

@@ -37,6 +37,7 @@
 #include <unordered_map>
 #include <string.h>
 #include "scc_internal.cuh"
+#include "scc_record.cuh"
 
 struct ServerRequest {
     int64_t id = 0;
@@ -59,7 +60,8 @@ struct ServerSession {
 struct scc_server {
     int device = 0;
     int64_t budget = 0;
-    int64_t in_use = 0;          // resident sessions + admitted requests
+    int64_t in_use = 0;          // resident sessions + admitted requests + drain scratch
+    int64_t drain_reserved = 0;  // the drain scratch in in_use; a request that fits without it waits, it is not refused
     std::mutex mu;
     std::condition_variable cv_work, cv_done;
     std::vector<ServerSession> sessions;
@@ -156,13 +158,29 @@ static int64_t update_bytes(int32_t n, int64_t m, int64_t k_ins, int64_t k_del) 
     return 10LL * (m + k_ins) + 64LL * (k_ins + k_del) + 16LL * (int64_t)n + (1 << 20);
 }
 
+// The record drain's scratch is reserved while a request runs, for the most
+// vertices that can be live.  Where the budget has no room for it the request
+// is admitted all the same and keeps to the plain drain, which takes none.
+// Both under the lock.
+static int64_t reserve_drain_scratch(scc_server* sv, int32_t n) {
+    const int64_t bytes = scc_record_bytes(n);
+    if (sv->in_use + bytes > sv->budget) return 0;
+    sv->in_use += bytes;
+    sv->drain_reserved += bytes;
+    return bytes;
+}
+static void release_drain_scratch(scc_server* sv, int64_t bytes) {
+    sv->in_use -= bytes;
+    sv->drain_reserved -= bytes;
+}
+
 static void worker_main(scc_server* sv) {
     cudaSetDevice(sv->device);
     for (;;) {
         ServerRequest* r = nullptr;
         ServerSession* ses = nullptr;
         std::vector<ServerRequest*> grp;
-        int64_t grp_bytes = 0;
+        int64_t grp_bytes = 0, scratch = 0;
         {
             std::unique_lock<std::mutex> lk(sv->mu);
             for (;;) {
@@ -187,7 +205,8 @@ static void worker_main(scc_server* sv) {
                         break;
                     }
                     if (sv->in_use + c->est_bytes > sv->budget) {
-                        if (sv->inflight == 0) {   // can never fit: reject
+                        // can never fit: reject
+                        if (sv->inflight == 0 && sv->in_use - sv->drain_reserved + c->est_bytes > sv->budget) {
                             c->rc = SCC_ERR_OOM;
                             c->done = true;
                             c->t_done = now_ms();
@@ -232,6 +251,8 @@ static void worker_main(scc_server* sv) {
             }
             ses->busy = true;
             sv->in_use += grp_bytes;
+            scratch = reserve_drain_scratch(sv, ses->g->n);
+            ses->s->drain_scratch = scratch;
             sv->inflight++;
             sv->max_inflight = std::max(sv->max_inflight, sv->inflight);
             double t0 = now_ms();
@@ -254,6 +275,7 @@ static void worker_main(scc_server* sv) {
             double t1 = now_ms();
             ses->busy = false;
             sv->in_use -= grp_bytes;
+            release_drain_scratch(sv, scratch);
             sv->in_use -= ses->resident;
             ses->resident = graph_bytes(ses->g->n, ses->g->m) + state_bytes(ses->g->n);
             sv->in_use += ses->resident;
@@ -309,23 +331,37 @@ extern "C" int scc_server_create(int device, int num_slots, int64_t hbm_budget_b
 // Takes ownership of g; decomposes it (method 2) before the session serves.
 extern "C" int scc_server_add_graph(scc_server* sv, scc_graph* g, int32_t* session) {
     SCC_REQUIRE(sv && g && session, SCC_ERR_INVALID, "NULL argument");
-    int64_t need = graph_bytes(g->n, g->m) + state_bytes(g->n);
+    int64_t need = graph_bytes(g->n, g->m) + state_bytes(g->n), scratch = 0;
     {
-        std::lock_guard<std::mutex> lk(sv->mu);
+        std::unique_lock<std::mutex> lk(sv->mu);
+        // room that only running requests' drain scratch takes is waited for
+        sv->cv_done.wait(lk, [&] {
+            return sv->in_use + need <= sv->budget || sv->in_use - sv->drain_reserved + need > sv->budget;
+        });
         SCC_REQUIRE(sv->in_use + need <= sv->budget, SCC_ERR_OOM, "graph needs %lld bytes, budget left %lld",
                     (long long)need, (long long)(sv->budget - sv->in_use));
         sv->in_use += need;
+        scratch = reserve_drain_scratch(sv, g->n);
     }
     scc_state* s = nullptr;
     int rc = scc_state_create(g, &s);
     scc_run_stats st;
-    if (rc == SCC_OK) rc = scc_run(g, s, SCC_METHOD_GLOBAL_WCC_FB, SCC_PIVOT_DEGREE, &st);
-    std::lock_guard<std::mutex> lk(sv->mu);
+    if (rc == SCC_OK) {
+        s->drain_scratch = scratch;
+        rc = scc_run(g, s, SCC_METHOD_GLOBAL_WCC_FB, SCC_PIVOT_DEGREE, &st);
+    }
+    {
+        std::lock_guard<std::mutex> lk(sv->mu);
+        release_drain_scratch(sv, scratch);
+        if (rc != SCC_OK) sv->in_use -= need;
+    }
+    sv->cv_done.notify_all();
+    sv->cv_work.notify_all();
     if (rc != SCC_OK) {
-        sv->in_use -= need;
         scc_state_free(s);
         return rc;
     }
+    std::lock_guard<std::mutex> lk(sv->mu);
     ServerSession ses;
     ses.g = g; ses.s = s; ses.resident = need;
     sv->sessions.push_back(ses);
