@@ -236,6 +236,7 @@ __device__ void b_peel(const BatchArgs& a, int32_t* q, int32_t* qc, int32_t* s_t
 // 4,096 graphs, 63.8 M vertices, 383 M edges, default shape: 23.7 ms with
 // colours and marks in global memory and the peel first, 3.7 ms so (sweeps
 // from a sixteenth on 3.8 ms, from half on 4.4 ms).
+#define B_MARKS_MAX (200 * 1024) // vertices of the largest graph whose marks are kept so, a byte each
 #define B_BLOCK_DEG 512          // top-down lists longer than this are expanded by the whole block
 #define B_BIG 64                 // such items one level sets aside (further ones: by their warp)
 #define B_SWEEP 4                // sweep once the frontier (both directions) is this share of the vertices not reached
@@ -695,7 +696,7 @@ struct scc_batch_plan {
     int32_t* d_live2 = nullptr;
     int32_t* d_ctr = nullptr;
     int32_t* h_ctr = nullptr;
-    int32_t max_n = 0;          // vertices of the largest graph
+    int32_t marks_n = 0;        // vertices of the largest graph whose marks fit shared memory
     scc_batch_tuning tune;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -717,15 +718,16 @@ static int batch_enqueue(scc_batch_plan* p, int sms) {
     a.ctr = p->d_ctr;
     a.warp_deg = p->tune.warp_deg;
     a.members = nullptr;
-    // Marks of the largest graph, up to 200 KB (204,800 vertices); larger graphs
-    // take the rounds over global marks from the start.  Where the marks leave
-    // fewer blocks resident than asked for, the others follow: no block waits
-    // for another.
-    const int32_t smem = std::min(200 * 1024, (p->max_n + 3) & ~3);
+    // Marks of the largest graph that fits B_MARKS_MAX; larger graphs take the
+    // rounds over global marks from the start and ask for none: 300 graphs of 210,000
+    // vertices on one block an SM with 200 KB each take 79 ms, on two
+    // without 47.  Where the marks leave fewer blocks resident than asked
+    // for, the others follow: no block waits for another.
+    const int32_t smem = (p->marks_n + 3) & ~3;
     a.marks_cap = smem;
     a.vec_adj = ((reinterpret_cast<uintptr_t>(g->node_idx) | reinterpret_cast<uintptr_t>(g->r_node_idx)) & 15u) == 0;
     a.adj_len = g->m;
-    SCC_CUDA(cudaFuncSetAttribute(k_batch_scc, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    SCC_CUDA(cudaFuncSetAttribute(k_batch_scc, cudaFuncAttributeMaxDynamicSharedMemorySize, B_MARKS_MAX));
     SCC_CUDA(cudaMemsetAsync(p->d_ctr, 0, sizeof(int32_t) * BATCH_CTR_WORDS, s->stream));
     k_batch_scc<<<sms * p->tune.blocks_per_sm, p->tune.threads, smem, s->stream>>>(a);
     SCC_CUDA(cudaPeekAtLastError());
@@ -769,7 +771,10 @@ extern "C" int scc_batch_plan_create(const scc_graph* g, scc_state* s, const int
     SCC_CUDA(cudaSetDevice(s->device));
     scc_batch_plan* p = new scc_batch_plan();
     p->g = g; p->s = s; p->G = num_graphs;
-    for (int32_t i = 0; i < num_graphs; ++i) p->max_n = std::max(p->max_n, offsets[i + 1] - offsets[i]);
+    for (int32_t i = 0; i < num_graphs; ++i) {
+        const int32_t ng = offsets[i + 1] - offsets[i];
+        if (ng <= B_MARKS_MAX) p->marks_n = std::max(p->marks_n, ng);
+    }
     if (tuning) p->tune = *tuning; else scc_batch_default_tuning(&p->tune);
     if (!batch_tuning_ok(&p->tune)) { delete p; scc_set_error("bad batch tuning"); return SCC_ERR_INVALID; }
     cudaEventCreate(&p->ev[0]); cudaEventCreate(&p->ev[1]);
