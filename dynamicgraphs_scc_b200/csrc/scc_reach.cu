@@ -501,6 +501,11 @@ __global__ void __launch_bounds__(REACH_THREADS) k_reach_bottomup(RoundArgs a, i
 #define COOP_BLOCK_EDGES 65536       // list entries of the graph, both directions, per block of a small round
 #define COOP_NARROW 12               // narrow levels run here before the plain drain takes over
 #define COOP_WAIT_LIMIT (1 << 24)
+// Levels after which the host goes on: the barrier counts its arrivals in 32
+// bits, two barriers a level.  Only a chain walked with the drains tuned away gets there.
+#define COOP_LEVELS (1 << 18)
+#define COOP_BLOCKS 2048             // most blocks of a launch
+static_assert((2LL * COOP_LEVELS + 4) * COOP_BLOCKS < (1LL << 31), "barrier arrivals");
 #define COOP_MAX_DEGREE 128          // mean degree up to which the chunk list fits its buffer
 // control words (one 128-byte line each where blocks poll or add)
 #define CC_BAR 0
@@ -757,7 +762,7 @@ __global__ void __launch_bounds__(REACH_THREADS, 4) k_round_coop(RoundArgs a, Co
         which ^= 1;
         n = next;
         narrow = (!bottom_up && next <= c.async_max && edges_small) ? narrow + 1 : 0;
-        if (n > 0 && (falling || (narrow > 0 && pays) || narrow >= COOP_NARROW)) { code = 1; break; }
+        if (n > 0 && (falling || (narrow > 0 && pays) || narrow >= COOP_NARROW || level >= COOP_LEVELS)) { code = 1; break; }
     }
     if (code == 0 && c.mode != COOP_REACH) {
         // classification, as k_classify
@@ -1124,7 +1129,7 @@ static int coop_blocks(int device, int64_t live, int64_t m) {
     // 148, 0.22 level by level from the host), so the graph's own edges count too.
     const int64_t want = std::max<int64_t>(std::max<int64_t>(8, (live + 63) / 64), 2 * m / COOP_BLOCK_EDGES);
     const int64_t cap = live > (1 << 17) ? (int64_t)sms * per : sms;
-    return (int)std::min(want, cap);
+    return (int)std::min<int64_t>(std::min(want, cap), COOP_BLOCKS);
 }
 
 int scc_impl_round_coop(const scc_graph* g, scc_state* s, RoundArgs& a, int mode, bool one_class, bool compact,
