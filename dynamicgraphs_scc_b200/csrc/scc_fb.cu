@@ -293,7 +293,7 @@ int scc_impl_fb_round(const scc_graph* g, scc_state* s, int32_t only_color, int3
 // components (so independent pieces get their own pivot), then one FW-BW
 // round over all classes at once.  Every class loses at least its pivot's SCC
 // per round, so the loop ends.
-int scc_impl_resolve_all(const scc_graph* g, scc_state* s, bool classes_split) {
+int scc_impl_resolve_all(const scc_graph* g, scc_state* s, bool as_they_are) {
     if (s->live_count < 0) SCC_TRY(scc_impl_compact_live(g, s, true));
     double t_round = scc_trace_on() ? trace_ms() : 0.0;
     for (int round = 0; round < (1 << 30); ++round) {
@@ -306,10 +306,11 @@ int scc_impl_resolve_all(const scc_graph* g, scc_state* s, bool classes_split) {
             SCC_TRY(scc_impl_resolve_tail(g, s, &taken));
             if (taken) break;
         }
-        if (round == 0 && classes_split) {
-            // the caller peeled to the fixpoint, compacted, then split: a split
-            // only recolours weakly disconnected parts, so no live vertex loses
-            // a same-colour neighbour and this round's peel would find nothing
+        if (round == 0 && as_they_are) {
+            // either the caller peeled to the fixpoint, compacted, then split -- a
+            // split only recolours weakly disconnected parts, so no live vertex
+            // loses a same-colour neighbour and a peel would find nothing -- or an
+            // update left old SCCs, whose trimmable vertices the next round peels
             classes = -1;
         } else {
             SCC_TRY(scc_impl_trim1(g, s, true, &t));

@@ -206,8 +206,9 @@ cudaError_t scc_impl_malloc_async(void** p, size_t bytes, cudaStream_t st);
 bool scc_impl_take_wait_injection();   // consumes a pending SCC_INJECT_WAIT
 int scc_impl_take_idle_injection();    // consumes a pending SCC_INJECT_IDLE: polls, 0 = none
 void scc_impl_pivot_release(scc_state* s);   // frees the learned-pivot and logging buffers
-// classes_split: the live classes are already weak components (a split ran last)
-int scc_impl_resolve_all(const scc_graph* g, scc_state* s, bool classes_split = false);
+// as_they_are: the first round takes the live classes without a peel and a split
+// (they ran last, or the classes are an update's old SCCs; any colouring is right)
+int scc_impl_resolve_all(const scc_graph* g, scc_state* s, bool as_they_are = false);
 // Decomposes every remaining class in one launch (a block per class); *taken is
 // false, with nothing done, when a class is above tune.tail_class vertices.
 int scc_impl_resolve_tail(const scc_graph* g, scc_state* s, bool* taken);

@@ -30,6 +30,7 @@
 //    SCC_DEVERR_WAIT_LIMIT and returns, and the host reports SCC_ERR_TIMEOUT.
 #include <stdlib.h>
 #include <algorithm>
+#include <atomic>
 #include "scc_round.cuh"
 #include "scc_tile.cuh"
 #include "scc_record.cuh"
@@ -495,7 +496,7 @@ __global__ void __launch_bounds__(REACH_THREADS) k_reach_bottomup(RoundArgs a, i
 // Values that other blocks wrote in this launch are read past L1 (__ldcg,
 // volatile): queues, counters, chunk lists, slots, marks.  Colours and CSR do
 // not change before the classification, which only reads its own vertices.
-#define COOP_CHUNK 1024              // entries of one chunk (at least; more on graphs of that mean degree)
+#define COOP_CHUNK 1024              // entries of one chunk
 #define COOP_DEG 256                 // lists longer than this are cut into chunks
 #define COOP_LANE_CHUNKS 8           // a list of more chunks is entered by its warp, not by its lane
 #define COOP_BLOCK_EDGES 65536       // list entries of the graph, both directions, per block of a small round
@@ -506,7 +507,10 @@ __global__ void __launch_bounds__(REACH_THREADS) k_reach_bottomup(RoundArgs a, i
 #define COOP_LEVELS (1 << 18)
 #define COOP_BLOCKS 2048             // most blocks of a launch
 static_assert((2LL * COOP_LEVELS + 4) * COOP_BLOCKS < (1LL << 31), "barrier arrivals");
-#define COOP_MAX_DEGREE 128          // mean degree up to which the chunk list fits its buffer
+// Mean degree m / n up to which a level's chunk list fits its 2 n + 64 entries: lists
+// above COOP_DEG are at most 2 m / 256 <= n, their chunks at most 2 m / 1024 <= n / 4 more.
+#define COOP_MAX_DEGREE 128
+static_assert(2 * COOP_MAX_DEGREE <= COOP_DEG && 2 * COOP_MAX_DEGREE <= COOP_CHUNK, "chunk list");
 // control words (one 128-byte line each where blocks poll or add)
 #define CC_BAR 0
 #define CC_Q 32                      // three rotating frontier lengths, a line each
@@ -517,7 +521,6 @@ static_assert(CC_EDGES + 96 <= CTR_COOP_WORDS, "control words");
 struct CoopArgs {
     int32_t* q[2];
     int32_t* chunk_item; long long* chunk_at;
-    int32_t chunk;
     int32_t* cc;
     int32_t mode;                    // COOP_ROUND, COOP_SEEDED or COOP_REACH
     int32_t one_class;
@@ -679,12 +682,12 @@ __global__ void __launch_bounds__(REACH_THREADS, 4) k_round_coop(RoundArgs a, Co
                 const int32_t d = valid ? __ldg(off + v + 1) - __ldg(off + v) : 0;
                 int32_t m = 0, at = 0;
                 if (d > COOP_DEG) {
-                    m = (d + c.chunk - 1) / c.chunk;
+                    m = (d + COOP_CHUNK - 1) / COOP_CHUNK;
                     at = atomicAdd(cc + CC_CHUNKS + 32 * o, m);
                     if (m <= COOP_LANE_CHUNKS) {
                         for (int32_t j = 0; j < m; ++j) {
                             c.chunk_item[at + j] = it;
-                            c.chunk_at[at + j] = (long long)j * c.chunk;
+                            c.chunk_at[at + j] = (long long)j * COOP_CHUNK;
                         }
                     }
                     valid = false;
@@ -697,7 +700,7 @@ __global__ void __launch_bounds__(REACH_THREADS, 4) k_round_coop(RoundArgs a, Co
                     const int32_t lit = __shfl_sync(full, it, l);
                     for (int32_t j = lane; j < lm; j += 32) {
                         c.chunk_item[lat + j] = lit;
-                        c.chunk_at[lat + j] = (long long)j * c.chunk;
+                        c.chunk_at[lat + j] = (long long)j * COOP_CHUNK;
                     }
                 }
                 expand_warp(a, valid, it, push);
@@ -712,7 +715,7 @@ __global__ void __launch_bounds__(REACH_THREADS, 4) k_round_coop(RoundArgs a, Co
                     const int32_t* off = dir ? a.r_begin : a.begin;
                     const int32_t* adj = dir ? a.r_node_idx : a.node_idx;
                     const int32_t b = __ldg(off + v) + (int32_t)__ldcg(c.chunk_at + x);
-                    const int32_t len = min(__ldg(off + v + 1) - b, c.chunk);
+                    const int32_t len = min(__ldg(off + v + 1) - b, COOP_CHUNK);
                     const int32_t col = __ldg(a.color + v);
                     const unsigned bit = 1u << dir;
                     for (int32_t k0 = 0; k0 < len; k0 += 4 * REACH_THREADS) {
@@ -1112,16 +1115,17 @@ static bool tile_round(scc_state* s, int32_t* lo, int32_t* hi) {
 // bottom-up while the frontier holds more than 2*live/bu_div items.
 
 static int coop_blocks(int device, int64_t live, int64_t m) {
-    static int cached_sms[64] = {0}, cached_per[64] = {0};
+    static std::atomic<int> cached[64];      // SMs << 8 | resident blocks an SM
     int sms = 148, per = 1;
-    if (device >= 0 && device < 64 && cached_sms[device]) {
-        sms = cached_sms[device];
-        per = cached_per[device];
+    const int known = device >= 0 && device < 64 ? cached[device].load() : 0;
+    if (known) {
+        sms = known >> 8;
+        per = known & 255;
     } else {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_round_coop, REACH_THREADS, 0);
         if (per < 1) per = 1;
-        if (device >= 0 && device < 64) { cached_per[device] = per; cached_sms[device] = sms; }
+        if (device >= 0 && device < 64) cached[device] = sms << 8 | per;
     }
     // A barrier costs more with more blocks: a small round takes one block an SM
     // or fewer.  Few live vertices may still hold most of a large graph's edges (19
@@ -1140,7 +1144,6 @@ int scc_impl_round_coop(const scc_graph* g, scc_state* s, RoundArgs& a, int mode
     CoopArgs c;
     c.q[0] = s->qa; c.q[1] = s->qb;
     c.chunk_item = s->hq; c.chunk_at = s->hoff;
-    c.chunk = (int32_t)std::max<int64_t>(COOP_CHUNK, 2 * g->m / std::max<int32_t>(g->n, 1) + 1);
     c.cc = s->ctr + CTR_MAX;
     c.mode = mode;
     c.one_class = one_class ? 1 : 0;
