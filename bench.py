@@ -67,13 +67,15 @@ WORKLOAD_NAMES = {
 }
 
 
-# DRAM traffic of the record drain relative to its algorithmic bytes, from one
-# ncu capture (dram__bytes_read.sum + dram__bytes_write.sum over all launches)
-# of `bench.py --workload grid4096 --steps 1 --warmup 0`: 965.55 MB read +
-# written by 4 launches whose algorithmic bytes total 1,014.27 MB.  The
-# full C2 step is too large for that capture; its drain runs the same grid.
-ASYNC_TRAFFIC_RATIO = 965.55 / 1014.27
-ASYNC_TRAFFIC_SOURCE = "ncu dram bytes on the 4096x4096 grid workload (0.952 x algorithmic), scaled per launch"
+# The two drains of narrow frontiers, by the ledger's setting that times them: kernel, algorithmic bytes
+# of its items and edges, and DRAM traffic relative to those bytes from one ncu capture (dram__bytes_read.sum +
+# dram__bytes_write.sum over all launches) of one decomposition of the grid4096 workload.  The
+# full C2 step is too large for that capture; its drains run the same grid.
+#   record drain: 32 B per expanded record, 4 B per claim (one atomic on a mark)
+#   plain drain:  13 B per expanded item (offset pair, colour, mark), 9 B per scanned edge (neighbour
+#                 id, its colour, its mark)
+DRAINS = {2: ("k_reach_records", 32, 4, 967.01 / 769.04),
+          1: ("k_reach_async", 13, 9, 595.40 / 793.8)}
 
 
 def measured_peak_gbs():
@@ -886,10 +888,15 @@ def main():
     def timed(mode, sampler=None):
         """W untimed steps, then K steps bracketed by barrier + synchronize and
         CUDA events on the state's stream; max over ranks."""
-        for _ in range(args.warmup):
+        capi.call("scc_state_profile", st.handle, 2)
+        for _ in range(max(args.warmup, 1)):
             st.reset()
             st.run(2, mode)
         st.synchronize()
+        l_ms, l_launch, l_items, l_edges = C.c_double(), C.c_int64(), C.c_int64(), C.c_int64()
+        ledger_args = (C.byref(l_ms), C.byref(l_launch), C.byref(l_items), C.byref(l_edges))
+        capi.call("scc_state_profile_read", st.handle, *ledger_args)
+        drain = 2 if l_launch.value > 0 else 1
         if sampler is not None:
             sampler.start()
         barrier()
@@ -898,7 +905,7 @@ def main():
         ev1 = torch.cuda.Event(enable_timing=True)
         kernels = 0
         phase = []
-        capi.call("scc_state_profile", st.handle, 1)   # time the dominant kernel's launches on this stream
+        capi.call("scc_state_profile", st.handle, drain)   # time the dominant kernel's launches on this stream
         ev0.record(stream)
         for _ in range(args.steps):
             st.reset()
@@ -910,12 +917,10 @@ def main():
         torch.cuda.synchronize()
         barrier()
         clocks = sampler.stop() if sampler is not None else None
-        l_ms, l_launch, l_items, l_edges = C.c_double(), C.c_int64(), C.c_int64(), C.c_int64()
-        capi.call("scc_state_profile_read", st.handle, C.byref(l_ms), C.byref(l_launch), C.byref(l_items),
-                  C.byref(l_edges))
+        capi.call("scc_state_profile_read", st.handle, *ledger_args)
         capi.call("scc_state_profile", st.handle, 0)
         ms, _ = reduce_replicas(ev0.elapsed_time(ev1) / args.steps, m, dist, f"cuda:{local_rank}")
-        return ms, kernels, phase, clocks, (l_ms, l_launch, l_items, l_edges)
+        return ms, kernels, phase, clocks, (drain, l_ms, l_launch, l_items, l_edges)
 
     plain = None
     if learned:                                 # the plain-pivot form on the same GPU, for the comparison
@@ -924,7 +929,7 @@ def main():
         plain = {"value": round(m * world / (p_ms * 1e-3) / 1e9, 4), "unit": "GTEPS", "ms_per_step": round(p_ms, 4),
                  "fb_rounds": p_phase[-1]["fb_rounds"], "traversal_steps": p_phase[-1]["traversal_steps"]}
     ms, kernels, phase, clocks, ledger = timed(pivot_mode, ClockSampler(local_rank))
-    l_ms, l_launch, l_items, l_edges = ledger
+    drain, l_ms, l_launch, l_items, l_edges = ledger
     if learned and rank == 0:
         plain["labels_equal_learned"] = bool(np.array_equal(plain_labels, st.canonical_labels()))
     _, total_edges = reduce_replicas(ms, m, dist, f"cuda:{local_rank}")
@@ -934,17 +939,18 @@ def main():
     peak, peak_kind = measured_peak_gbs()
     b_alg = 16 * m + 20 * n + 8
     achieved = b_alg / (ms * 1e-3) / 1e9
-    # dominant kernel: the record drain (the plain drain's launches count with
-    # it where a round takes that one).  Algorithmic bytes: 13 B per expanded item (offset pair, colour, mark) + 9 B per scanned edge
-    # (neighbour id, its colour, its mark).
+    # dominant kernel: the record drain, or the plain drain where no round takes that one
     kernel_roofline = None
     if l_launch.value > 0 and l_ms.value > 0:
-        k_bytes = (13 * l_items.value + 9 * l_edges.value) / l_launch.value
+        k_name, per_item, per_edge, traffic = DRAINS[drain]
+        k_bytes = (per_item * l_items.value + per_edge * l_edges.value) / l_launch.value
         k_ms = l_ms.value / l_launch.value
         k_ach = k_bytes / (k_ms * 1e-3) / 1e9
-        kernel_roofline = {"bound": "hbm", "kernel": "k_reach_records", "achieved": round(k_ach, 2), "peak": peak,
+        kernel_roofline = {"bound": "hbm", "kernel": k_name, "achieved": round(k_ach, 2), "peak": peak,
                            "peak_kind": peak_kind, "unit": "GB/s", "frac": round(k_ach / peak, 5),
-                           "traffic": int(ASYNC_TRAFFIC_RATIO * k_bytes), "traffic_source": ASYNC_TRAFFIC_SOURCE,
+                           "traffic": int(traffic * k_bytes),
+                           "traffic_source": f"ncu dram bytes on the 4096x4096 grid workload ({traffic:.3f} x "
+                                             "algorithmic), scaled per launch",
                            "bytes_per_launch": int(k_bytes), "ms_per_launch": round(k_ms, 4),
                            "launches": l_launch.value, "share_of_step": round(l_ms.value / (ms * args.steps), 4)}
 

@@ -166,7 +166,7 @@ struct scc_state {
 
     // kernel ledger (scc_state_profile): device time and algorithmic bytes of
     // the asynchronous reachability drain, timed with events on `stream`
-    bool ledger_on = false;
+    int ledger_on = 0;               // 1: every drain, 2: the record drain alone
     cudaEvent_t lev[2];
     double ledger_ms = 0.0;
     long long ledger_launches = 0;

@@ -1254,13 +1254,13 @@ int scc_impl_reach(const scc_graph* g, scc_state* s, RoundArgs& a, int32_t qlen,
             SCC_TRY(scc_zero_counters(s, CTR_ASYNC_ITEMS, 4));
             SCC_TRY(scc_zero_counters(s, CTR_ABAIL, 1));
             a.async_bail = std::max<int32_t>(8 * s->tune.async_max, 1 << 16);
-            if (s->ledger_on) SCC_CUDA(cudaEventRecord(s->lev[0], s->stream));
+            if (s->ledger_on == 1) SCC_CUDA(cudaEventRecord(s->lev[0], s->stream));
             k_reach_async<<<async_blocks(s->device, s->tune.async_blocks_per_sm), ASYNC_THREADS, 0, s->stream>>>(a, s->aq, qcap);
             SCC_LAUNCHED(s);
-            if (s->ledger_on) SCC_CUDA(cudaEventRecord(s->lev[1], s->stream));
+            if (s->ledger_on == 1) SCC_CUDA(cudaEventRecord(s->lev[1], s->stream));
             s->traversal_steps++;
             SCC_TRY(scc_sync_counters(s));
-            if (s->ledger_on) {
+            if (s->ledger_on == 1) {
                 float ms = 0.f;
                 SCC_CUDA(cudaEventElapsedTime(&ms, s->lev[0], s->lev[1]));
                 s->ledger_ms += ms;

@@ -456,7 +456,7 @@ extern "C" int scc_state_set_tuning(scc_state* s, const scc_tuning* t) {
 
 extern "C" int scc_state_profile(scc_state* s, int enable) {
     SCC_REQUIRE(s, SCC_ERR_INVALID, "state is NULL");
-    s->ledger_on = enable != 0;
+    s->ledger_on = enable == 2 ? 2 : enable != 0;
     s->ledger_ms = 0.0;
     s->ledger_launches = s->ledger_items = s->ledger_edges = 0;
     return SCC_OK;

@@ -523,13 +523,13 @@ int scc_impl_reach_tile(const scc_graph* g, scc_state* s, RoundArgs& a, const in
         SCC_CUDA(cudaFuncSetAttribute(k_reach_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM_BYTES));
         attr_set[s->device] = true;
     }
-    if (s->ledger_on) SCC_CUDA(cudaEventRecord(s->lev[0], s->stream));
+    if (s->ledger_on == 1) SCC_CUDA(cudaEventRecord(s->lev[0], s->stream));
     k_reach_tile<<<t.ntiles, TILE_THREADS, TILE_SMEM_BYTES, s->stream>>>(a, t);
     SCC_LAUNCHED(s);
-    if (s->ledger_on) SCC_CUDA(cudaEventRecord(s->lev[1], s->stream));
+    if (s->ledger_on == 1) SCC_CUDA(cudaEventRecord(s->lev[1], s->stream));
     s->traversal_steps++;
     SCC_TRY(scc_sync_counters(s));
-    if (s->ledger_on) {
+    if (s->ledger_on == 1) {
         float ms = 0.f;
         SCC_CUDA(cudaEventElapsedTime(&ms, s->lev[0], s->lev[1]));
         s->ledger_ms += ms;

@@ -162,8 +162,9 @@ int scc_state_device_arrays(scc_state* s, int32_t** d_color, int32_t** d_scc);
 /* Kernel ledger (no counterpart in the reference; its phase timers are
  * gettimeofday, src/scc_main.cc:180-184): when enabled, every launch of the
  * asynchronous reachability drain is timed with CUDA events on the state's
- * stream and its work counted (items expanded, edges scanned).  Enabling or
- * disabling resets the totals. */
+ * stream and its work counted (items expanded, edges scanned; for the record
+ * drain, records expanded and vertices claimed or found claimed).  enable: 1 = every
+ * drain, 2 = the record drain alone, 0 = off.  Enabling or disabling resets the totals. */
 int scc_state_profile(scc_state* s, int enable);
 int scc_state_profile_read(scc_state* s, double* ms, int64_t* launches, int64_t* items, int64_t* edges);
 
