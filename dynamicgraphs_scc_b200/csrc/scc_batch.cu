@@ -231,8 +231,9 @@ __device__ void b_peel(const BatchArgs& a, int32_t* q, int32_t* qc, int32_t* s_t
 // memory, and the round comes before the peel, which then only sees what the
 // round left.  Narrow frontiers are expanded top down from the queue; from a
 // quarter of the vertices on, a sweep over all vertices takes over, whose
-// offsets and lists are read in order.  Bound by instruction issue and by the
-// round trips of narrow levels.
+// offsets and lists are read in order.  Bound by the barriers and the round trips
+// of its levels, and by instruction issue (43 % of the slots on 512 graphs; DRAM
+// 1.55 TB/s).
 // 4,096 graphs, 63.8 M vertices, 383 M edges, default shape: 23.7 ms with
 // colours and marks in global memory and the peel first, 3.7 ms so (sweeps
 // from a sixteenth on 3.8 ms, from half on 4.4 ms).
@@ -307,7 +308,7 @@ __device__ __forceinline__ bool b_probe_long(const FirstRound& r, uint32_t bit, 
 // costs what the one before it left.  A lane per vertex, two aligned int4
 // chunks of each direction's list in flight at once (a list of six entries is
 // then done in one round trip after its offsets), a list left at its first hit.
-// Bound by instruction issue and the round trips of a vertex's loads.  On the
+// Bound by the round trips of a vertex's loads and by instruction issue.  On the
 // batch named above: 3.7 ms; all vertices in every sweep 4.4 ms; the
 // lists of 32 vertices read end to end, a row of 32 entries at a time 5.7 ms; one
 // chunk and one direction at a time 7.1 ms.

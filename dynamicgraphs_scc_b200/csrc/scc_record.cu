@@ -33,7 +33,8 @@
 // vertex of more than REC_W class neighbours, or of a neighbour outside the live
 // list, has a LONG record: the warp that takes it walks its adjacency list with
 // the colour test; a claimed neighbour outside the live list goes to the host's
-// next frontier.
+// next frontier, as such a vertex does that is in the frontier already.  What a warp
+// shares after the idle ones gave up their tickets is collected by the host.
 #include <algorithm>
 #include "scc_record.cuh"
 

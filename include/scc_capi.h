@@ -191,7 +191,8 @@ typedef struct scc_tuning {
     int32_t tail_class;           /* ... provided no class has more vertices than this (1024) */
     int32_t cta_deg;              /* top-down items above this degree (up to huge_deg) are expanded by a whole
                                      block, their adjacency staged in shared memory by bulk copies; negative =
-                                     never */
+                                     never (256).  Only on graphs above 128 edges per vertex or with the tile
+                                     drain: other rounds run in one launch, which cuts lists into chunks */
 } scc_tuning;
 int scc_state_get_tuning(scc_state* s, scc_tuning* t);
 /* Fields <= 0 keep their current value, except tile_min_live, tail_live and
