@@ -235,8 +235,8 @@ __device__ void b_peel(const BatchArgs& a, int32_t* q, int32_t* qc, int32_t* s_t
 // of its levels, and by instruction issue (43 % of the slots on 512 graphs; DRAM
 // 1.55 TB/s).
 // 4,096 graphs, 63.8 M vertices, 383 M edges, default shape: 23.7 ms with
-// colours and marks in global memory and the peel first, 3.7 ms so (sweeps
-// from a sixteenth on 3.8 ms, from half on 4.4 ms).
+// colours and marks in global memory and the peel first, 3.35 ms so (3.7 without
+// B_LEAF; then, sweeps from a sixteenth on 3.8 ms, from half on 4.4 ms).
 #define B_MARKS_MAX (200 * 1024) // vertices of the largest graph whose marks are kept so, a byte each
 #define B_BLOCK_DEG 512          // top-down lists longer than this are expanded by the whole block
 #define B_BIG 64                 // such items one level sets aside (further ones: by their warp)
@@ -244,15 +244,22 @@ __device__ void b_peel(const BatchArgs& a, int32_t* q, int32_t* qc, int32_t* s_t
 #define B_STEP 8                 // entries of a short list claimed together
 #define B_PROBES 8               // two-chunk probes a lane makes alone before the warp takes the list
 
+// A vertex without out- or without in-edges is a component by itself and on no path
+// between others; the pass that finds the pivot sees its degrees and sets it aside.  Without
+// this, batches of acyclic and very sparse graphs paid for the first round on top of the
+// peel: 5,000 random graphs of 1,000 vertices and 500 edges 0.72 ms, 0.61 with the peel first,
+// 0.53 so; 1,000 binary trees of 8,191 0.64, 0.55 and 0.43; the batch below 3.35 ms.
+#define B_LEAF 4u
+
 struct FirstRound {
-    volatile uint8_t* marks;     // bit 0 FW reached, bit 1 BW reached, of vertex lo + i
+    volatile uint8_t* marks;     // of vertex lo + i: bit 0 FW reached, bit 1 BW reached, B_LEAF
     int32_t lo, ng;
 };
 
 // An id outside the graph (a batch whose graphs are not closed) is not claimed.
 __device__ __forceinline__ bool b_claim(const FirstRound& r, int dir, int32_t u) {
     const uint32_t i = (uint32_t)(u - r.lo), bit = 1u << dir;
-    if (i >= (uint32_t)r.ng || (r.marks[i] & bit)) return false;
+    if (i >= (uint32_t)r.ng || (r.marks[i] & (bit | B_LEAF))) return false;
     const uint32_t sh = (i & 3u) * 8u;
     return !((atomicOr(reinterpret_cast<uint32_t*>(const_cast<uint8_t*>(r.marks) + (i & ~3u)), bit << sh) >> sh) & bit);
 }
@@ -309,7 +316,7 @@ __device__ __forceinline__ bool b_probe_long(const FirstRound& r, uint32_t bit, 
 // chunks of each direction's list in flight at once (a list of six entries is
 // then done in one round trip after its offsets), a list left at its first hit.
 // Bound by the round trips of a vertex's loads and by instruction issue.  On the
-// batch named above: 3.7 ms; all vertices in every sweep 4.4 ms; the
+// batch named above (before B_LEAF): 3.7 ms; all vertices in every sweep 4.4 ms; the
 // lists of 32 vertices read end to end, a row of 32 entries at a time 5.7 ms; one
 // chunk and one direction at a time 7.1 ms.
 __device__ void b_sweep(const BatchArgs& a, const FirstRound& r, const int32_t* list, int32_t n, int32_t* open,
@@ -321,7 +328,8 @@ __device__ void b_sweep(const BatchArgs& a, const FirstRound& r, const int32_t* 
         const bool in = at0 + lane < n;
         const int32_t i = !in ? 0 : list ? list[at0 + lane] : at0 + lane;
         const int32_t v = r.lo + i;
-        const uint32_t had = in ? r.marks[i] : 3u;
+        uint32_t had = in ? r.marks[i] : 3u;
+        if (had & B_LEAF) had = 3u;
         int32_t k0 = 0, e0 = 0, k1 = 0, e1 = 0;
         if (!(had & 1u)) { k0 = __ldg(a.rbegin + v); e0 = __ldg(a.rbegin + v + 1); }
         if (!(had & 2u)) { k1 = __ldg(a.begin + v); e1 = __ldg(a.begin + v + 1); }
@@ -457,6 +465,7 @@ __device__ int32_t b_first_round(const BatchArgs& a, int32_t lo, int32_t ng, int
     for (int32_t i = threadIdx.x; i < ng; i += blockDim.x) {
         const unsigned long long k = pivot_key(a.begin, a.rbegin, lo + i);
         best = k > best ? k : best;
+        if (k >> 32 == 1u) r.marks[i] = B_LEAF;          // in x out is 0
     }
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long y = __shfl_xor_sync(full, best, o);
@@ -500,9 +509,11 @@ __device__ int32_t b_first_round(const BatchArgs& a, int32_t lo, int32_t ng, int
     __syncthreads();
     for (int32_t i0 = threadIdx.x - lane; i0 < ng; i0 += blockDim.x) {
         const int32_t i = i0 + lane, v = lo + i;
-        const uint32_t m = i < ng ? r.marks[i] : 3u;
+        uint32_t m = i < ng ? r.marks[i] : 3u;
+        const bool leaf = (m & B_LEAF) != 0u;
+        if (leaf) m = 3u;
         if (i < ng) {
-            a.scc[v] = m == 3u ? p : SCC_NIL_NODE;
+            a.scc[v] = m == 3u ? (leaf ? v : p) : SCC_NIL_NODE;
             a.color[v] = m == 3u ? SCC_COLOR_DONE : m == 1u ? b_fw_colour(p) : m == 2u ? b_bw_colour(p) : c0;
             if (m != 3u) a.mark[v] = 0;
         }
