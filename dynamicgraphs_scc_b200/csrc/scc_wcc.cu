@@ -215,11 +215,11 @@ __device__ __forceinline__ uint32_t uf_rank(int32_t x) {
 // a root (the compare-and-swap sees memory, not L1) to a vertex of higher
 // rank, root or not: ranks rise along parents, so no link closes a cycle, and
 // the vertex of highest rank stays the component's root.
-// The finds stand at the head of the loop, so that the lanes of a warp meet
-// there before each compare-and-swap.  With the first two before the loop and the
-// others at its end, lanes retried one after another where a warp walks a hub's
-// list: method 0 on R-MAT s18 (2 M edges) 1.8-2.1 ms and up to 2.6 from call to call, 1.00
-// so, and s24 29-45 ms, 26.0 so (every find past L1: 1.2 and 31.5 ms).
+// For a warp on a hub's list: the finds stand at the head of the loop, so that
+// its lanes meet there before each compare-and-swap.  With the first two before the
+// loop and the others at its end the lanes retried one after another: method 0 on
+// R-MAT s18 (2 M edges) 1.8-2.1 ms and up to 2.6 from call to call, 0.97 so, and
+// s24 29-45 ms, 25.7 so (every find past L1: 1.2 and 31.5 ms).
 __device__ __forceinline__ int32_t uf_union(int32_t* __restrict__ uf, int32_t a, int32_t b) {
     for (bool fresh = false;; fresh = true) {
         a = fresh ? uf_find<true>(uf, a) : uf_find<false>(uf, a);
@@ -228,6 +228,21 @@ __device__ __forceinline__ int32_t uf_union(int32_t* __restrict__ uf, int32_t a,
         const int32_t lo = uf_rank(a) < uf_rank(b) ? a : b, hi = lo == a ? b : a;
         if (atomicCAS(uf + lo, lo, hi) == lo) return hi;
         a = lo; b = hi;
+    }
+}
+
+// The same for a lane on its own short list, whose finds rarely end together: it need
+// not wait for the others there (a union of 4,096 random graphs, 64 M vertices: 14.7 ms
+// for its split, 15.8 with the form above).
+__device__ __forceinline__ int32_t uf_union_lane(int32_t* __restrict__ uf, int32_t a, int32_t b) {
+    a = uf_find<false>(uf, a);
+    b = uf_find<false>(uf, b);
+    for (;;) {
+        if (a == b) return a;
+        const int32_t lo = uf_rank(a) < uf_rank(b) ? a : b, hi = lo == a ? b : a;
+        if (atomicCAS(uf + lo, lo, hi) == lo) return hi;
+        a = uf_find<true>(uf, lo);
+        b = uf_find<true>(uf, hi);
     }
 }
 
@@ -283,7 +298,7 @@ __global__ void k_uf_hook(const int32_t* __restrict__ begin, const int32_t* __re
                 for (int j = 0; j < 4; ++j) par[j] = w[j] != v ? uf_parent<false>(uf, w[j]) : v;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (w[j] != v && col[j] == c) rv = uf_union(uf, rv, par[j]);
+                    if (w[j] != v && col[j] == c) rv = uf_union_lane(uf, rv, par[j]);
             }
         }
     }
