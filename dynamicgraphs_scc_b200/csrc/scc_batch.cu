@@ -232,8 +232,8 @@ __device__ void b_peel(const BatchArgs& a, int32_t* q, int32_t* qc, int32_t* s_t
 // round left.  Narrow frontiers are expanded top down from the queue; from a
 // quarter of the vertices on, a sweep over all vertices takes over, whose
 // offsets and lists are read in order.  Bound by the barriers and the round trips
-// of its levels, and by instruction issue (43 % of the slots on 512 graphs; DRAM
-// 1.55 TB/s).
+// of its levels, and by instruction issue (44 % of the slots on 512 graphs; DRAM
+// 1.49 TB/s).
 // 4,096 graphs, 63.8 M vertices, 383 M edges, default shape: 23.7 ms with
 // colours and marks in global memory and the peel first, 3.35 ms so (3.7 without
 // B_LEAF; then, sweeps from a sixteenth on 3.8 ms, from half on 4.4 ms).
