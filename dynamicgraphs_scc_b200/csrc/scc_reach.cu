@@ -501,7 +501,9 @@ __global__ void __launch_bounds__(REACH_THREADS) k_reach_bottomup(RoundArgs a, i
 #define COOP_LANE_CHUNKS 8           // a list of more chunks is entered by its warp, not by its lane
 #define COOP_BLOCK_EDGES 65536       // list entries of the graph, both directions, per block of a small round
 #define COOP_NARROW 12               // narrow levels run here before the plain drain takes over
-#define COOP_WAIT_LIMIT (1 << 24)
+// Polls of a barrier before it gives up, about 0.7 us each: blocks wait for the
+// slowest thread of a sweep, which may read one list of hundreds of millions of entries alone.
+#define COOP_WAIT_LIMIT (1 << 27)
 // Levels after which the host goes on: the barrier counts its arrivals in 32
 // bits, two barriers a level.  Only a chain walked with the drains tuned away gets there.
 #define COOP_LEVELS (1 << 18)
